@@ -497,6 +497,44 @@ __global__ void __launch_bounds__(128) embedding_scatter_add_kernel(const float*
     }
 }
 
+// ── row gather and transpose of fp32 matrices ──
+// Pure copies, bound by HBM. PyTorch's strided copy_ runs a scalar index-computing kernel for both
+// patterns (a carried memory = the last state of every trajectory, 512 rows of 16 KB one trajectory
+// apart: 8 + 8 MB; tied embeddings, 512 x 8192 transposed: 17 + 17 MB).
+__global__ void __launch_bounds__(256) copy_rows_kernel(const float4* __restrict__ src, long long src_stride4,
+                                                        float4* __restrict__ dst, int row4, int per_row)
+{
+    // per_row CTAs share a row, four independent 16-byte loads in flight per thread
+    const long long r = blockIdx.x / per_row;
+    const int part = (int)(blockIdx.x % per_row);
+    const float4* s = src + r * src_stride4;
+    float4* d = dst + r * (long long)row4;
+    for (int i = part * 1024 + threadIdx.x; i < row4; i += per_row * 1024) {
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (i + u * 256 < row4) v[u] = s[i + u * 256];
+#pragma unroll
+        for (int u = 0; u < 4; u++) if (i + u * 256 < row4) d[i + u * 256] = v[u];
+    }
+}
+constexpr int TR_TILE = 64;
+// 64 x 64 tiles through shared memory: 256-byte segments on both sides; the odd leading dimension
+// keeps the column reads free of bank conflicts.
+__global__ void __launch_bounds__(256) transpose_kernel(const float* __restrict__ src, float* __restrict__ dst,
+                                                        int rows, int cols)
+{
+    __shared__ float t[TR_TILE][TR_TILE + 1];
+    const int r0 = blockIdx.y * TR_TILE, c0 = blockIdx.x * TR_TILE;
+    const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
+#pragma unroll
+    for (int i = 0; i < TR_TILE; i += 4)
+        if (r0 + ty + i < rows && c0 + tx < cols) t[ty + i][tx] = src[(size_t)(r0 + ty + i) * cols + c0 + tx];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TR_TILE; i += 4)
+        if (c0 + ty + i < cols && r0 + tx < rows) dst[(size_t)(c0 + ty + i) * rows + r0 + tx] = t[tx][ty + i];
+}
+
 }  // namespace nlh
 
 using namespace nlh;
@@ -746,6 +784,32 @@ int32_t nlh_cross_entropy_backward(const void* logits, int32_t logits_is_bf16, c
     else
         ce_bwd_kernel<float><<<n, 256, 0, st>>>((const float*)logits, target_ids, lse, grad_scale, (float*)d_logits, vocab, inv_count);
     return check_launch("nlh_cross_entropy_backward") ? NLH_OK : NLH_ERR_CUDA;
+}
+
+int32_t nlh_copy_rows(const float* src, int64_t src_stride, float* dst, int32_t rows, int32_t row_len)
+{
+    if (rows < 0 || row_len < 0 || src_stride < 0 || !src || !dst) return NLH_ERR_INVALID_ARG;
+    if (rows == 0 || row_len == 0) return NLH_OK;
+    if ((((uintptr_t)src | (uintptr_t)dst) & 15) || (src_stride & 3) || (row_len & 3)) {
+        const cudaError_t e = cudaMemcpy2DAsync(dst, (size_t)row_len * 4, src, (size_t)src_stride * 4, (size_t)row_len * 4,
+                                                rows, cudaMemcpyDeviceToDevice, current_stream());
+        if (e != cudaSuccess) record_status(NLH_ERR_CUDA, "nlh_copy_rows", cudaGetErrorString(e));
+        return e == cudaSuccess ? NLH_OK : NLH_ERR_CUDA;
+    }
+    const int row4 = row_len >> 2, per_row = (row4 + 1023) / 1024;
+    copy_rows_kernel<<<(unsigned)rows * per_row, 256, 0, current_stream()>>>(
+        (const float4*)src, src_stride >> 2, (float4*)dst, row4, per_row);
+    return check_launch("nlh_copy_rows") ? NLH_OK : NLH_ERR_CUDA;
+}
+
+int32_t nlh_transpose(const float* src, float* dst, int32_t rows, int32_t cols)
+{
+    if (rows < 0 || cols < 0 || !src || !dst) return NLH_ERR_INVALID_ARG;
+    if (rows == 0 || cols == 0) return NLH_OK;
+    const dim3 grid((cols + TR_TILE - 1) / TR_TILE, (rows + TR_TILE - 1) / TR_TILE);
+    if (grid.y > 65535) return NLH_ERR_INVALID_ARG;
+    transpose_kernel<<<grid, 256, 0, current_stream()>>>(src, dst, rows, cols);
+    return check_launch("nlh_transpose") ? NLH_OK : NLH_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -19,20 +19,23 @@ import torch
 from . import ffi
 
 RULE_DELTA, RULE_TITANS, RULE_HEBBIAN = 0, 1, 2
-_PROTOS = None
+_PLANS = {}      # entry name -> (function, ((argument, is pointer), ...), return type)
 
 
-def _protos():
-    global _PROTOS
-    if _PROTOS is None:
-        _PROTOS = ffi.parse_header()
-    return _PROTOS
+def _plan(name):
+    """Call plan of a C-ABI entry: the prototype is parsed and the symbol looked up once."""
+    ret, argtypes, argnames = ffi.prototypes()[name]
+    plan = _PLANS[name] = (getattr(ffi.lib(), name), tuple((an, at is C.c_void_p) for an, at in zip(argnames, argtypes)),
+                           ret)
+    return plan
 
 
 def bind_stream(stream: torch.cuda.Stream | None = None) -> None:
     """Point the library at a torch stream (default: torch's current stream)."""
-    s = stream if stream is not None else torch.cuda.current_stream()
-    ffi.lib().nlh_set_stream(C.c_void_p(s.cuda_stream))
+    if stream is not None:
+        ffi.lib().nlh_set_stream(stream.cuda_stream)
+    else:                                # the raw handle: no Stream object is built on every call
+        ffi.lib().nlh_set_stream(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def call(name: str, **kw):
@@ -42,34 +45,30 @@ def call(name: str, **kw):
     None as NULL. Status-returning entries are checked; void entries are checked
     through the library's recorded status.
     """
-    ret, argtypes, argnames = _protos()[name]
-    missing = [a for a in argnames if a not in kw]
-    extra = [a for a in kw if a not in argnames]
-    if missing or extra:
-        raise TypeError(f"{name}: missing {missing}, unexpected {extra}")
-    args = []
-    for an, at in zip(argnames, argtypes):
-        v = kw[an]
-        if at is C.c_void_p:
-            if v is None:
-                args.append(C.c_void_p(0))
-            elif isinstance(v, torch.Tensor):
+    fn, params, ret = _PLANS.get(name) or _plan(name)
+    try:
+        args = [kw[an] for an, _ in params]
+    except KeyError:
+        args = ()
+    if len(args) != len(kw):
+        names = [an for an, _ in params]
+        raise TypeError(f"{name}: missing {[a for a in names if a not in kw]}, "
+                        f"unexpected {[a for a in kw if a not in names]}")
+    # the loader set argtypes: ctypes converts integers (pointers included), floats and None itself
+    for i, v in enumerate(args):
+        if isinstance(v, torch.Tensor):
+            an, is_ptr = params[i]
+            if is_ptr:
                 if not v.is_cuda or not v.is_contiguous():
                     raise ValueError(f"{name}.{an}: need a contiguous CUDA tensor")
-                args.append(C.c_void_p(v.data_ptr()))
-            elif isinstance(v, int):
-                args.append(C.c_void_p(v))
-            else:
-                args.append(v)
-        else:
-            args.append(at(v))
-    fn = getattr(ffi.lib(), name)
+                args[i] = v.data_ptr()
     bind_stream()
     if ret is None:
         ffi.lib().nlh_clear_status()   # void entries report through the recorded status
     rc = fn(*args)
     if ret is C.c_int32:
-        ffi.check(rc, name)
+        if rc:
+            ffi.check(rc, name)
     elif ret is C.c_uint32:
         if rc != 0:
             raise RuntimeError(f"{name}: cudaError {rc}")

@@ -65,6 +65,15 @@ def parse_header(path: str = HEADER):
 
 
 _lib = None
+_protos = None
+
+
+def prototypes():
+    """parse_header() of this library's header, parsed once."""
+    global _protos
+    if _protos is None:
+        _protos = parse_header()
+    return _protos
 
 
 def lib() -> C.CDLL:
@@ -76,7 +85,7 @@ def lib() -> C.CDLL:
                 f"{LIB_PATH} is missing: build it with `python -m nl_hecate_b200.build` "
                 "(there is no CPU fallback)")
         handle = C.CDLL(LIB_PATH)
-        for name, (ret, argtypes, _) in parse_header().items():
+        for name, (ret, argtypes, _) in prototypes().items():
             fn = getattr(handle, name)   # AttributeError if the header and library disagree
             fn.restype = ret
             fn.argtypes = argtypes

@@ -13,14 +13,15 @@ post-update clamp (``b_theta`` in [-10, 2]).
 """
 from __future__ import annotations
 
-import ctypes as C
-
+import numpy as np
 import torch
 
 from . import ffi
 from .dispatch import call
 
 CHUNK = 8192  # elements per CTA work item
+RING = 4      # steps of descriptors that may be in flight
+_DESC = np.dtype(ffi.AdamWTensorDesc)
 
 
 class FlatAdamW:
@@ -47,56 +48,81 @@ class FlatAdamW:
         self.chunk_tensor = torch.tensor(ct, dtype=torch.int32, device=dev)
         self.chunk_start = torch.tensor(cs, dtype=torch.int64, device=dev)
         self.chunk_len = torch.tensor(cl, dtype=torch.int32, device=dev)
-        self._desc_host = (ffi.AdamWTensorDesc * len(self.sizes))()
-        nbytes = C.sizeof(self._desc_host)
-        self._desc_pinned = torch.empty(nbytes, dtype=torch.uint8)
+        # Per-tensor descriptors of one step. The columns that stay are written once into every row of
+        # the ring. The table travels through a small ring of pinned host rows: prepare() fills the
+        # next one while the GPU may still have to read the previous ones, so the host runs ahead of
+        # the device.
+        nt = len(self.sizes)
+        base = np.zeros(nt, dtype=_DESC)
+        self._row_decay = [None] * RING
+        for i, (lo, hi) in self.clamp.items():
+            base["clamp_lo"][i], base["clamp_hi"][i], base["has_clamp"][i] = lo, hi, 1
+        pinned = torch.empty(RING, nt * _DESC.itemsize, dtype=torch.uint8)
         if dev.type == "cuda":
-            self._desc_pinned = self._desc_pinned.pin_memory()
-        self._desc_dev = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+            pinned = pinned.pin_memory()
+        self._desc_ring = pinned
+        self._desc_rows = pinned.numpy().view(_DESC)
+        self._desc_rows[:] = base
+        self._desc_dev = torch.empty(nt * _DESC.itemsize, dtype=torch.uint8, device=dev)
         self._partial = torch.empty(148 * 8, dtype=torch.float32, device=dev)
         self.norm = torch.zeros(1, dtype=torch.float32, device=dev)
         self.scale = torch.ones(1, dtype=torch.float32, device=dev)
-        # recorded after the stream-ordered upload of the pinned table in launch(); prepare()
-        # waits on it before it rewrites the table, so a host that runs ahead of the GPU cannot
+        # one event per ring row, recorded after the stream-ordered upload of that row; prepare()
+        # waits on it before it rewrites the row, so a host that runs ahead of the GPU cannot
         # replace step t's descriptors before step t's copy has read them
-        self._uploaded = torch.cuda.Event() if dev.type == "cuda" else None
-        self._upload_pending = False
+        self._uploaded = [torch.cuda.Event() for _ in range(RING)] if dev.type == "cuda" else None
+        self._row_busy = [False] * RING
+        self._row = 0
+        self._captured_row = None      # set when a graph captured the upload of a row: that row is then reused
+        self._prepared = False
 
     def view(self, arena: torch.Tensor, i: int) -> torch.Tensor:
         o, n = self.slices[i]
         return arena[o:o + n]
 
     def prepare(self, steps, active=None, lr_scale=1.0):
-        """Host part of a step: fill the per-tensor descriptor table (bias corrections from each
-        tensor's own 1-based step count, activity, clamp, learning-rate scale) in pinned memory.
-        The device reads it in launch(); a second prepare() first waits until the previous
-        launch()'s upload of the table has completed."""
-        if self._upload_pending:
-            self._uploaded.synchronize()
-            self._upload_pending = False
-        nt = len(self.sizes)
-        active = [True] * nt if active is None else active
-        for i in range(nt):
-            d = self._desc_host[i]
-            t = max(int(steps[i]), 1)
-            d.bc1_inv = 1.0 / (1.0 - self.beta1 ** t)
-            d.bc2_inv = 1.0 / (1.0 - self.beta2 ** t)
-            d.weight_decay = 0.0 if i in self.no_decay else self.weight_decay
-            d.lr_scale = lr_scale
-            lo, hi = self.clamp.get(i, (0.0, 0.0))
-            d.clamp_lo, d.clamp_hi, d.has_clamp = lo, hi, int(i in self.clamp)
-            d.active = int(bool(active[i]))
-        C.memmove(self._desc_pinned.data_ptr(), C.addressof(self._desc_host),
-                  C.sizeof(self._desc_host))
+        """Host part of a step: fill the next row of the descriptor ring (bias corrections from each
+        tensor's own 1-based step count, activity, learning-rate scale). The device reads it after
+        upload(); a row is rewritten only when the upload that last used it has completed."""
+        r = self._row = (self._row + 1) % RING if self._captured_row is None else self._captured_row
+        if self._row_busy[r]:
+            self._uploaded[r].synchronize()
+            self._row_busy[r] = False
+        row = self._desc_rows[r]
+        t = np.maximum(np.asarray(steps, dtype=np.int64), 1)
+        if (t == t[0]).all():                    # one count for all tensors: one power per moment
+            t = t[:1]
+        row["bc1_inv"] = 1.0 / (1.0 - self.beta1 ** t.astype(np.float64))
+        row["bc2_inv"] = 1.0 / (1.0 - self.beta2 ** t.astype(np.float64))
+        row["lr_scale"] = lr_scale
+        if self.weight_decay != self._row_decay[r]:
+            row["weight_decay"] = self.weight_decay
+            row["weight_decay"][list(self.no_decay)] = 0.0
+            self._row_decay[r] = self.weight_decay
+        row["active"] = True if active is None else np.asarray(active, dtype=bool)
+        self._prepared = True
+
+    def upload(self):
+        """Stream-ordered copy of the prepared descriptors to the device. launch() does it itself;
+        a caller that replays a captured launch() calls it before the capture and before every
+        replay, so that the graph holds no copy from a fixed host row."""
+        r = self._row
+        self._desc_dev.copy_(self._desc_ring[r], non_blocking=True)
+        if self._uploaded is None:
+            pass
+        elif torch.cuda.is_current_stream_capturing():
+            self._captured_row = r
+        else:
+            self._uploaded[r].record()
+            self._row_busy[r] = True
+        self._prepared = False
 
     def launch(self, lr, max_grad_norm=0.0):
-        """Device part of a step (stream-ordered, capturable in a CUDA graph): descriptor upload,
-        global-norm clip scale, multi-tensor AdamW. Returns the device scalar with the pre-clip
-        gradient norm (valid only when max_grad_norm > 0)."""
-        self._desc_dev.copy_(self._desc_pinned, non_blocking=True)
-        if self._uploaded is not None and not torch.cuda.is_current_stream_capturing():
-            self._uploaded.record()
-            self._upload_pending = True
+        """Device part of a step (stream-ordered, capturable in a CUDA graph): upload of descriptors
+        that are not on the device yet, global-norm clip scale, multi-tensor AdamW. Returns the device
+        scalar with the pre-clip gradient norm (valid only when max_grad_norm > 0)."""
+        if self._prepared:
+            self.upload()
         scale_ptr = None
         if max_grad_norm > 0.0:
             call("nlh_arena_grad_norm_clip", g=self.g, n=self.arena_len,

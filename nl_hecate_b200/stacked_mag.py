@@ -133,7 +133,8 @@ class _TitansMemory(torch.autograd.Function):
         if carry is not None:
             # the carried memory is updated in place from the last stored state (one strided copy;
             # the kernels have read m0 by then, stream order), no separate m_final tensor
-            carry.copy_(ms[:, -1])
+            n, slots, dd = ms.shape
+            D.call("nlh_copy_rows", src=ms[:, -1].data_ptr(), src_stride=slots * dd, dst=carry, rows=n, row_len=dd)
             return y, None
         m_final = ms[:, -1].clone()
         ctx.mark_non_differentiable(m_final)
@@ -1034,8 +1035,12 @@ class StackedMAG:
         cfg = self.cfg
         self.opt.launch(cfg.lr, cfg.max_grad_norm)
         if cfg.tie_embeddings:
-            with torch.no_grad():   # gpu_stacked_sync_embed_weights: w_embed <- w_unembed^T
-                self.p["w_embed"].copy_(self.p["w_unembed"].t())
+            # gpu_stacked_sync_embed_weights: w_embed <- w_unembed^T
+            if self.device.type == "cuda":
+                D.call("nlh_transpose", src=self.p["w_unembed"], dst=self.p["w_embed"], rows=cfg.d_model, cols=cfg.vocab)
+            else:
+                with torch.no_grad():
+                    self.p["w_embed"].copy_(self.p["w_unembed"].t())
         self.opt.g.zero_()
 
     def apply_update(self):
@@ -1068,6 +1073,7 @@ class StackedMAG:
             torch.cuda.synchronize()
             torch.cuda.empty_cache()
             self._host_schedule()
+            self.opt.upload()
             self._graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(self._graph):
                 self._static_loss = self.forward_backward(self._static_tok, self._static_tgt,
@@ -1075,15 +1081,14 @@ class StackedMAG:
                 self.sync_gradients(process_group, world)
                 self._device_update()
             self._graph.replay()            # capture records only: run the scheduled step now
-            self._graph_done = torch.cuda.Event()
-            self._graph_done.record()
             return self._static_loss
         self._static_tok.copy_(tokens, non_blocking=True)
         self._static_tgt.copy_(targets, non_blocking=True)
-        self._graph_done.synchronize()      # the previous replay has consumed the descriptors
+        # the descriptors go to the device ahead of the replay, stream-ordered: the host does not wait
+        # for the previous step and its bookkeeping runs while the GPU is still busy with it
         self._host_schedule()
+        self.opt.upload()
         self._graph.replay()
-        self._graph_done.record()
         return self._static_loss
 
     def n_params(self):
