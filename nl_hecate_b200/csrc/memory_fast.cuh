@@ -747,8 +747,6 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
 }
 
 // ───────────────────────────── host dispatch ─────────────────────────────
-inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
-
 inline bool fast_common_ok(int d, float clip, float mmax)
 {
     return (d == 64 || d == 32) && !(clip > 0.0f) && !m_norm_enabled(mmax);

@@ -6,7 +6,7 @@
 // dimension and options allow it, the generic-d kernels otherwise.
 #include "memory_generic.cuh"
 #include "memory_exact_bwd.cuh"
-#include "chunk_mm.cuh"
+#include "memory_tc.h"
 #include "../../include/nlh_ffi.h"
 
 namespace nlh {
@@ -67,7 +67,7 @@ static int run_forward(int rule, FwdArgs a, const char* where)
         return NLH_ERR_INVALID_ARG;
     }
     cudaStream_t st = current_stream();
-    if (option_value(NLH_OPT_CHUNK_MATRIX) && cmm::forward(rule, a, st))
+    if (option_value(NLH_OPT_CHUNK_MATRIX) && mtc::forward(rule, a, a.frozen ? a.interval : 1, st))
         return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (fast_forward(rule, a, st)) return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (rule == RULE_TITANS && a.s_out == nullptr) {
@@ -92,6 +92,16 @@ static int run_forward(int rule, FwdArgs a, const char* where)
     return ok ? NLH_OK : NLH_ERR_CUDA;
 }
 
+// Backward in matrix form on the tensor cores. Stored states: chunk / checkpoint boundaries (a.chunk
+// tokens apart) or every state, of which only one per tile is read. A tile costs about as much as 24
+// tokens of the per-token kernels, whatever its length: shorter ranges stay with those.
+static bool tile_backward(int rule, const BwdArgs& a, cudaStream_t st)
+{
+    const long long dd = (long long)a.d * a.d;
+    if (a.chunk > 0) return mtc::backward(rule, a, a.chunk, a.frozen ? a.chunk : 1, dd, st);
+    return !a.frozen && a.t_end - a.t_start >= 24 && mtc::backward(rule, a, 64, 1, 64 * dd, st);
+}
+
 static int run_backward(int rule, BwdArgs a, const char* where)
 {
     if (!valid_dims(where, a.seq_len, a.d, a.batch)) return NLH_ERR_INVALID_ARG;
@@ -101,7 +111,7 @@ static int run_backward(int rule, BwdArgs a, const char* where)
         return NLH_ERR_INVALID_ARG;
     }
     cudaStream_t st = current_stream();
-    if (option_value(NLH_OPT_CHUNK_MATRIX) && cmm::backward(rule, a, st))
+    if (option_value(NLH_OPT_CHUNK_MATRIX) && tile_backward(rule, a, st))
         return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (fast_backward(rule, a, st)) return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (rule == RULE_TITANS && a.s_traj == nullptr) {
@@ -663,7 +673,7 @@ int32_t nlh_bulk_timeout_flag(void)
 {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_bulk_timeout, sizeof(int)) != cudaSuccess) return -1;
-    return v;
+    return v != 0 ? v : mtc::timeout_flag();
 }
 
 }  // extern "C"

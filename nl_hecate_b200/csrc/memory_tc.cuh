@@ -1,0 +1,970 @@
+// Titans / Delta memory rule in CHUNK-PARALLEL (matrix) form on the 5th-generation tensor cores,
+// head dimension 64: exact rule, frozen-M0 rule, and frozen rule with several chunks per tile.
+//
+// A problem's tokens are cut into tiles of up to 64. Inside a tile everything is linear in the
+// tile-start state (M0, S0) and the errors E (rows e_t). With r_t = 1 - alpha_t and, for t >= j,
+//     h(j,t)  = prod_{i=j+1..t} eta_i ,  rho(j,t) = prod_{i=j+1..t} r_i
+//     Om(t,j) = sum_{i=j..t} h(j,i) rho(i,t)        (weight of -theta_j e_j k_j^T in the state M_t)
+//     A_t = prod_{i<=t} r_i,  H_t = prod_{i<=t} eta_i,  B_t = eta_0 Om(t,0)   (weights of M0, S0)
+//     W(t,j) = theta_j Om(t,j)
+// the state after token t is  M_t = A_t M0 + B_t S0 - sum_{j<=t} W(t,j) e_j k_j^T. The error of
+// token t is read from the state of index u(t): t-1 for the exact rule, the last token before its
+// chunk for the frozen rule (u = -1: the tile-start state). With a_t = A_u, b_t = B_u (1, 0 for u = -1)
+//     (I + Lx) E = diag(a) K M0^T + diag(b) K S0^T - V ,   Lx(t,j) = W(u(t),j) (k_t . k_j)
+//     Y   = diag(A) Q M0^T + diag(B) Q S0^T - (W o P) E ,  P = Q K^T
+//     M_C = A_L M0 + B_L S0 - E^T diag(W(L-1,:)) K ,       S_C = H_L S0 - E^T diag(theta_j h(j,L-1)) K
+// and backward (G_M, G_S: gradients of the tile-end states)
+//     (I + Lx)^T F = -[ (W o P)^T dY + diag(W(L-1,:)) K G_M^T + diag(theta h) K G_S^T ] ,  dV = -F
+//     R = dY E^T ,  N = F E^T ,  Z = -W(u,:) o N
+//     dQ  = diag(A) dY M0 + diag(B) dY S0 - (W o R) K
+//     dK  = diag(a) F M0 + diag(b) F S0 - diag(W(L-1,:)) E G_M - diag(theta h) E G_S + (Z + Z^T) K - (W o R)^T Q
+//     G_M' = dY^T diag(A) Q + F^T diag(a) K + A_L G_M
+//     G_S' = dY^T diag(B) Q + F^T diag(b) K + B_L G_M + H_L G_S
+// The gate gradients contract the states with their adjoints and reduce to two decayed scans down
+// the columns of X(s,j) = R(s,j) P(s,j) + sum_{t: u(t)=s} N(t,j) (k_t . k_j), plus two columns for M0
+// and S0. Only W's recurrences over tokens are sequential, and they are 64 scalar steps.
+// Same semantics as the per-token statements core/kernels/titans_forward.cu:83-199,
+// titans_backward.cu:66-345 and titans_chunkwise_{forward,backward}.cu.
+//
+// Precision. Operands are fp32 and stay so: each is stored as THREE bf16 planes x = hi + mid + lo,
+// which hold all 24 bits of the significand, and a product is the six plane products
+// hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi accumulated in fp32 in TMEM, the small ones first (the
+// dropped ones are below 2^-24 of the product). Triangular solves, scans and gate tables are fp32 FMA.
+//
+// What bounds it. One CTA (256 threads) walks one problem, so a launch is bound by the chain of a
+// tile's stages: tensor products (48 cycles per 128x64x16 plane product at the shared-memory read
+// rate), the conversion of every intermediate into planes, and the 64-row triangular solves.
+//
+// Shared-memory matrices: element (row, col) of an R-row plane at (col/8)*(R*16) + row*16 + (col%8)*2,
+// the canonical no-swizzle core-matrix layout with the 8-column chunk outermost. The same bytes serve
+// as K-major operand (rows = M/N index) and as MN-major operand (rows = contraction index), so no
+// transposed copy of anything exists. Every MMA has M = 128; where a product has 64 rows the other
+// 64 lanes compute garbage from whatever follows in shared memory and are never read.
+#pragma once
+
+#include "nlh_common.cuh"
+#include "tc_common.cuh"
+
+namespace nlh {
+namespace mtc {
+
+using namespace nlh::tc;
+
+constexpr int D = 64, DD = D * D;
+constexpr int TMAX = 64;          // tokens per tile
+constexpr int NT = 256;
+constexpr int LDX = 68;           // leading dimension of the fp32 solve buffers
+constexpr int LDS = 67;           // leading dimension of the scan buffers (64 columns + M0 + S0)
+constexpr unsigned TCOLS = 512;
+constexpr int MIN_TILE = 16;      // shorter tiles run the per-token register kernels
+
+__device__ int g_mtc_timeout = 0;
+
+// ── fp32 <-> three bf16 planes ──
+__device__ __forceinline__ unsigned pack2(float a, float b)
+{
+    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const unsigned*>(&t);
+}
+__device__ __forceinline__ float lo_f(unsigned p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float hi_f(unsigned p) { return __uint_as_float(p & 0xffff0000u); }
+// 8 consecutive columns (chunk cc) of one row
+__device__ __forceinline__ void store8(unsigned char* t, int R, int plane, int row, int cc, const float* v)
+{
+    unsigned h[4], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float x = v[2 * i], y = v[2 * i + 1];
+        h[i] = pack2(x, y);
+        const float x1 = x - lo_f(h[i]), y1 = y - hi_f(h[i]);
+        m[i] = pack2(x1, y1);
+        l[i] = pack2(x1 - lo_f(m[i]), y1 - hi_f(m[i]));
+    }
+    unsigned char* p = t + cc * (R * 16) + row * 16;
+    *reinterpret_cast<uint4*>(p) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(p + plane) = make_uint4(m[0], m[1], m[2], m[3]);
+    *reinterpret_cast<uint4*>(p + 2 * plane) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+__device__ __forceinline__ void load8(float* v, const unsigned char* t, int R, int plane, int row, int cc)
+{
+    const unsigned char* p = t + cc * (R * 16) + row * 16;
+    const uint4 h = *reinterpret_cast<const uint4*>(p);
+    const uint4 m = *reinterpret_cast<const uint4*>(p + plane);
+    const uint4 l = *reinterpret_cast<const uint4*>(p + 2 * plane);
+    const unsigned hh[4] = {h.x, h.y, h.z, h.w}, mm[4] = {m.x, m.y, m.z, m.w}, ll[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        v[2 * i] = (lo_f(ll[i]) + lo_f(mm[i])) + lo_f(hh[i]);
+        v[2 * i + 1] = (hi_f(ll[i]) + hi_f(mm[i])) + hi_f(hh[i]);
+    }
+}
+// 32 columns starting at chunk cc0
+__device__ __forceinline__ void store32(unsigned char* t, int R, int plane, int row, int cc0, const float (&v)[32])
+{
+#pragma unroll
+    for (int c = 0; c < 4; c++) store8(t, R, plane, row, cc0 + c, v + 8 * c);
+}
+
+// ── tensor product of split operands, issued by one thread ──
+// D[128, N] (+)= A B with contraction length 16 * ksteps. a_mn / b_mn: the operand's rows are the
+// contraction index (MN-major), otherwise its rows are the M / N index (K-major).
+template <bool AMN, bool BMN>
+__device__ __forceinline__ void mma6(unsigned d, unsigned a, int a_plane, int a_R, unsigned b, int b_plane, int b_R,
+                                     int N, int ksteps)
+{
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((AMN ? 1u : 0u) << 15) | ((BMN ? 1u : 0u) << 16) |
+                           ((unsigned)(N >> 3) << 17) | (8u << 24);
+    const uint64_t ab = AMN ? make_desc(0, 128, a_R * 16) : make_desc(0, a_R * 16, 128);
+    const uint64_t bb = BMN ? make_desc(0, 128, b_R * 16) : make_desc(0, b_R * 16, 128);
+    const unsigned as = AMN ? 256 : a_R * 32, bs = BMN ? 256 : b_R * 32;    // bytes per 16 contraction steps
+    unsigned acc = 0;
+#pragma unroll 1
+    for (int p = 0; p < 6; p++) {
+        // plane pairs (2,0) (0,2) (1,1) (1,0) (0,1) (0,0)
+        const unsigned pa = p == 0 ? 2u : (p == 2 || p == 3) ? 1u : 0u;
+        const unsigned pb = p == 1 ? 2u : (p == 2 || p == 4) ? 1u : 0u;
+        const unsigned a0 = a + pa * a_plane, b0 = b + pb * b_plane;
+#pragma unroll 4
+        for (int k = 0; k < ksteps; k++) {
+            mma_bf16(d, ab + ((a0 + k * as) >> 4), bb + ((b0 + k * bs) >> 4), idesc, acc);
+            acc = 1;
+        }
+    }
+}
+
+// ── gates of a tile ──
+struct Tables {
+    float4 gt[TMAX];            // r_t, eta_t, theta_t of the tile's tokens (padding: 1, 0, 0)
+    float wM[TMAX], wS[TMAX];   // W(L-1,j), theta_j h(j,L-1)
+    float tot[8];               // A_L, B_L, H_L
+    float z[4][2 * TMAX];       // backward: row dots of the two column halves (zM, zS, gm, gs)
+    float part[2][2 * TMAX];
+    float red[8][4];
+    unsigned long long bar[4];
+    unsigned tmem;
+};
+
+// Row u of W for this thread's 32 columns (half hf): w[i] = W(u, 32 hf + i), and A_u, B_u.
+__device__ __forceinline__ void decay_row(const float4* gt, int u, int hf, float (&w)[32], float& au, float& bu)
+{
+    float rho = 1.f, om = 1.f;
+    auto step = [&](int j) {       // from column j+1 to column j
+        const float4 g = gt[j + 1];
+        const bool in = j < u;
+        rho = in ? rho * g.x : 1.f;
+        om = in ? fmaf(g.y, om, rho) : 1.f;
+    };
+    w[31] = (63 <= u) ? gt[63].z : 0.f;
+#pragma unroll
+    for (int j = 62; j >= 32; j--) { step(j); w[j - 32] = (j <= u) ? gt[j].z * om : 0.f; }
+    if (hf == 0) {
+#pragma unroll
+        for (int j = 31; j >= 0; j--) { step(j); w[j] = (j <= u) ? gt[j].z * om : 0.f; }
+    } else {
+#pragma unroll
+        for (int j = 31; j >= 0; j--) step(j);
+    }
+    au = (u >= 0) ? rho * gt[0].x : 1.f;
+    bu = (u >= 0) ? om * gt[0].y : 0.f;
+}
+
+// X <- (I + Lo)^{-1} X and X <- (I + Lo)^{-T} X for the strictly lower triangular Lo [n16*16 rows],
+// X 64 columns, both fp32 with leading dimension LDX. Blocked by 16 rows: the diagonal block by
+// substitution (one thread per column), the rest as rank-16 updates over all threads.
+__device__ __forceinline__ void diag16(const float* __restrict__ Lo, float* X, int r0, int c)
+{
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = X[(r0 + i) * LDX + c];
+#pragma unroll
+    for (int i = 1; i < 16; i++) {
+        const float* row = Lo + (r0 + i) * LDX + r0;
+#pragma unroll
+        for (int j4 = 0; j4 < i; j4 += 4) {
+            const float4 l = *reinterpret_cast<const float4*>(row + j4);
+            x[i] = fmaf(-l.x, x[j4], x[i]);
+            if (j4 + 1 < i) x[i] = fmaf(-l.y, x[j4 + 1], x[i]);
+            if (j4 + 2 < i) x[i] = fmaf(-l.z, x[j4 + 2], x[i]);
+            if (j4 + 3 < i) x[i] = fmaf(-l.w, x[j4 + 3], x[i]);
+        }
+        X[(r0 + i) * LDX + c] = x[i];
+    }
+}
+__device__ __forceinline__ void diag16_t(const float* __restrict__ Lo, float* X, int r0, int c)
+{
+    float x[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) x[i] = X[(r0 + i) * LDX + c];
+#pragma unroll
+    for (int k = 15; k >= 1; k--) {
+        const float* row = Lo + (r0 + k) * LDX + r0;
+#pragma unroll
+        for (int j4 = 0; j4 < k; j4 += 4) {
+            const float4 l = *reinterpret_cast<const float4*>(row + j4);
+            x[j4] = fmaf(-l.x, x[k], x[j4]);
+            if (j4 + 1 < k) x[j4 + 1] = fmaf(-l.y, x[k], x[j4 + 1]);
+            if (j4 + 2 < k) x[j4 + 2] = fmaf(-l.z, x[k], x[j4 + 2]);
+            if (j4 + 3 < k) x[j4 + 3] = fmaf(-l.w, x[k], x[j4 + 3]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 15; i++) X[(r0 + i) * LDX + c] = x[i];
+}
+__device__ __forceinline__ void solve_lower(const float* __restrict__ Lo, float* X, int n16)
+{
+    const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
+    for (int b = 0; b < n16; b++) {
+        if (g == b) diag16(Lo, X, 16 * b, c);
+        __syncthreads();
+        if (b + 1 < n16) {
+            float x[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) x[k] = X[(16 * b + k) * LDX + c];
+            for (int i0 = 16 * (b + 1) + 4 * g; i0 < 16 * n16; i0 += 16) {
+                float s[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    float acc = X[(i0 + i) * LDX + c];
+                    const float* row = Lo + (i0 + i) * LDX + 16 * b;
+#pragma unroll
+                    for (int k4 = 0; k4 < 16; k4 += 4) {
+                        const float4 l = *reinterpret_cast<const float4*>(row + k4);
+                        acc = fmaf(-l.x, x[k4], acc); acc = fmaf(-l.y, x[k4 + 1], acc);
+                        acc = fmaf(-l.z, x[k4 + 2], acc); acc = fmaf(-l.w, x[k4 + 3], acc);
+                    }
+                    s[i] = acc;
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) X[(i0 + i) * LDX + c] = s[i];
+            }
+            __syncthreads();
+        }
+    }
+}
+__device__ __forceinline__ void solve_lower_t(const float* __restrict__ Lo, float* X, int n16)
+{
+    const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
+    for (int b = n16 - 1; b >= 0; b--) {
+        if (g == b) diag16_t(Lo, X, 16 * b, c);
+        __syncthreads();
+        if (b > 0) {
+            float x[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) x[k] = X[(16 * b + k) * LDX + c];
+            for (int i0 = 4 * g; i0 < 16 * b; i0 += 16) {
+                float s[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) s[i] = X[(i0 + i) * LDX + c];
+#pragma unroll
+                for (int k = 0; k < 16; k++) {
+                    const float4 l = *reinterpret_cast<const float4*>(Lo + (16 * b + k) * LDX + i0);
+                    s[0] = fmaf(-l.x, x[k], s[0]); s[1] = fmaf(-l.y, x[k], s[1]);
+                    s[2] = fmaf(-l.z, x[k], s[2]); s[3] = fmaf(-l.w, x[k], s[3]);
+                }
+#pragma unroll
+                for (int i = 0; i < 4; i++) X[(i0 + i) * LDX + c] = s[i];
+            }
+            __syncthreads();
+        }
+    }
+}
+
+__device__ __forceinline__ void ld32(float (&v)[32], const float* __restrict__ p, bool ok)
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const float4 x = ok ? *reinterpret_cast<const float4*>(p + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[4 * i] = x.x; v[4 * i + 1] = x.y; v[4 * i + 2] = x.z; v[4 * i + 3] = x.w;
+    }
+}
+__device__ __forceinline__ void st32(float* p, const float (&v)[32])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        *reinterpret_cast<float4*>(p + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+}
+__device__ __forceinline__ void tload(float (&v)[32], unsigned taddr)
+{
+    unsigned r[32];
+    tmem_ld_32x32b_x32(r, taddr);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = __uint_as_float(r[i]);
+}
+
+// Bounded wait on one of the CTA's barriers; each barrier is waited on once per commit.
+struct Waiter {
+    unsigned bar0, phases;
+    bool dead;
+    __device__ __forceinline__ void operator()(int i)
+    {
+        if (!dead) dead = !mbar_wait(bar0 + 8 * i, (phases >> i) & 1u, WAIT_LIMIT);
+        phases ^= 1u << i;
+        fence_after_sync();
+    }
+};
+// all generic-proxy writes to shared memory and TMEM reads so far are ordered before the MMAs that one
+// thread issues after it
+__device__ __forceinline__ void publish()
+{
+    fence_async_proxy();
+    fence_before_sync();
+    __syncthreads();
+}
+
+// ───────────────────────────────── forward ─────────────────────────────────
+constexpr int F_KQ = 0, F_MS = 49152, F_WP = 98304, F_E = 122880, F_EW = 147456, F_X = 196608;
+constexpr int F_TAB = F_X + TMAX * LDX * 4;
+constexpr int FWD_SMEM = F_TAB + (int)sizeof(Tables);
+
+// T tokens per tile; rd tokens per frozen chunk (1: exact rule, T: the whole tile is one frozen chunk).
+// States are stored at every tile start and after the last token.
+template <int RULE, bool SOLVE>
+__global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int rd)
+{
+    constexpr bool HAS_S = (RULE == RULE_TITANS);
+    extern __shared__ __align__(1024) unsigned char sm[];
+    Tables& tb = *reinterpret_cast<Tables*>(sm + F_TAB);
+    float* Xb = reinterpret_cast<float*>(sm + F_X);      // right-hand side, then E, fp32
+    float* Lb = reinterpret_cast<float*>(sm + F_E);      // Lx, fp32, until the solve is over
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int R = (warp & 3) * 32 + (tid & 31), hf = warp >> 2;     // TMEM lane, column half
+    const int tr = R & 63;                                          // token (or state row) of this thread
+    const bool krow = R < 64;                                       // K / M rows, else Q / S rows
+    const int b = blockIdx.x;
+    const float* xg = (krow ? a.k : a.q) + (size_t)b * a.in_stride_tok * D + hf * 32;
+    const float* vg = a.v + (size_t)b * a.in_stride_tok * D + hf * 32;
+    const float* alg = a.alpha + (size_t)b * a.in_stride_tok;
+    const float* thg = a.theta + (size_t)b * a.in_stride_tok;
+    const float* etg = HAS_S ? a.eta + (size_t)b * a.in_stride_tok : nullptr;
+    float* yg = a.y + (size_t)b * a.seq_len * D + hf * 32;
+    float* sg = (krow ? a.m_out : a.s_out);                         // this thread's state output
+    if (HAS_S || krow) sg += (size_t)b * a.out_stride + tr * D + hf * 32;
+    const int ntile = (a.seq_len + T - 1) / T;
+
+    if (tid == 0) { mbar_init(smem_u32(&tb.bar[0]), 1); mbar_init(smem_u32(&tb.bar[1]), 1); mbar_init(smem_u32(&tb.bar[2]), 1); }
+    if (warp == 0) tmem_alloc_cols(reinterpret_cast<unsigned char*>(&tb.tmem), TCOLS);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const unsigned tm = tb.tmem;
+    const unsigned trow = tm + ((unsigned)((warp & 3) * 32) << 16) + hf * 32;
+    Waiter wait{smem_u32(&tb.bar[0]), 0u, false};
+    const unsigned kq = smem_u32(sm + F_KQ), ms = smem_u32(sm + F_MS), wp = smem_u32(sm + F_WP), ep = smem_u32(sm + F_E),
+                   ew = smem_u32(sm + F_EW);
+
+    float st[32];                     // fp32 row of M (krow) or S
+    if (HAS_S || krow) {
+        ld32(st, (krow ? a.m_init : a.s_init) + (size_t)b * a.init_stride + tr * D + hf * 32, true);
+        store32(sm + F_MS, 128, 16384, R, hf * 4, st);
+        st32(sg, st);
+    }
+    float x[32], v[32], gal = 0.f, gth = 0.f, get = 0.f;
+    auto fetch = [&](int c) {         // this thread's rows and gates of tile c
+        const int t0 = c * T, L = min(T, a.seq_len - t0);
+        const bool ok = tr < L;
+        ld32(x, xg + (size_t)(t0 + tr) * D, ok);
+        if (krow) ld32(v, vg + (size_t)(t0 + tr) * D, ok);
+        if (tid < TMAX) {
+            gal = (tid < L) ? alg[t0 + tid] : 0.f;
+            gth = (tid < L) ? thg[t0 + tid] : 0.f;
+            get = (HAS_S && tid < L) ? etg[t0 + tid] : 0.f;
+        }
+    };
+    if (ntile > 0) fetch(0);
+
+    for (int c = 0; c < ntile; c++) {
+        const int t0 = c * T, L = min(T, a.seq_len - t0);
+        store32(sm + F_KQ, 128, 16384, R, hf * 4, x);
+        if (tid < TMAX) tb.gt[tid] = make_float4(1.0f - gal, get, gth, 0.f);
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<false, false>(tm, kq, 16384, 128, ms, 16384, 128, HAS_S ? 128 : 64, 4);     // K,Q x M0,S0
+            mma6<false, false>(tm + 128, kq, 16384, 128, kq, 16384, 128, 64, 4);             // K,Q x K
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        float w[32], au, bu;
+        const int u = krow ? (tr / rd) * rd - 1 : tr;
+        decay_row(tb.gt, u, hf, w, au, bu);
+        if (R == 64 + L - 1) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) tb.wM[hf * 32 + i] = w[i];
+            if (hf == 0) { tb.tot[0] = au; tb.tot[1] = bu; }
+        }
+        if (HAS_S && tid < TMAX) {
+            float hh = 1.f;
+            for (int i = L - 1; i > tid; i--) hh *= tb.gt[i].y;
+            tb.wS[tid] = (tid < L) ? tb.gt[tid].z * hh : 0.f;
+            if (tid == 0) tb.tot[2] = hh * tb.gt[0].y;
+        }
+        wait(0);
+        float acc[32], p[32];
+        tload(acc, trow);
+#pragma unroll
+        for (int i = 0; i < 32; i++) acc[i] *= au;
+        if (HAS_S) {
+            tload(p, trow + 64);
+#pragma unroll
+            for (int i = 0; i < 32; i++) acc[i] = fmaf(bu, p[i], acc[i]);
+        }
+        tload(p, trow + 128);
+        if (krow) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) acc[i] -= v[i];
+            st32(Xb + tr * LDX + hf * 32, acc);
+            if (SOLVE) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) p[i] *= w[i];
+                st32(Lb + tr * LDX + hf * 32, p);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; i++) p[i] *= -w[i];
+            store32(sm + F_WP, 64, 8192, tr, hf * 4, p);
+        }
+        if (c + 1 < ntile) fetch(c + 1);         // lands under the solve and the products
+        __syncthreads();
+        if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
+        {
+            // E and its tile-end weighted copies as planes
+            const int row = tid & 63, q = tid >> 6;
+            const float wm = tb.wM[row], wsv = HAS_S ? tb.wS[row] : 0.f;
+            float e[16], s[8];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
+                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
+            }
+#pragma unroll
+            for (int c8 = 0; c8 < 2; c8++) {
+                store8(sm + F_E, 64, 8192, row, 2 * q + c8, e + 8 * c8);
+#pragma unroll
+                for (int i = 0; i < 8; i++) s[i] = e[8 * c8 + i] * wm;
+                store8(sm + F_EW, 64, 16384, row, 2 * q + c8, s);
+                if (HAS_S) {
+#pragma unroll
+                    for (int i = 0; i < 8; i++) s[i] = e[8 * c8 + i] * wsv;
+                    store8(sm + F_EW, 64, 16384, row, 8 + 2 * q + c8, s);
+                }
+            }
+        }
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<true, true>(tm + 256, ew, 16384, 64, kq, 16384, 128, 64, 4);              // [Ew Es]^T K
+            mma_commit(smem_u32(&tb.bar[1]));
+            mma6<false, true>(tm + 192, wp - 1024, 8192, 64, ep, 8192, 64, 64, 4);         // rows 64..127: -(W o P) E
+            mma_commit(smem_u32(&tb.bar[2]));
+        }
+        // tile-end states while the outputs' product runs (the partner row is read before anyone
+        // overwrites the planes)
+        const float At = tb.tot[0], Bt = tb.tot[1], Ht = tb.tot[2];
+#pragma unroll
+        for (int i = 0; i < 32; i++) st[i] *= krow ? At : Ht;
+        if (HAS_S && krow) {
+#pragma unroll
+            for (int c8 = 0; c8 < 4; c8++) {
+                float s[8];
+                load8(s, sm + F_MS, 128, 16384, 64 + tr, hf * 4 + c8);
+#pragma unroll
+                for (int i = 0; i < 8; i++) st[8 * c8 + i] = fmaf(Bt, s[i], st[8 * c8 + i]);
+            }
+        }
+        wait(1);
+        tload(p, trow + 256);
+        __syncthreads();
+        if (HAS_S || krow) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) st[i] -= p[i];
+            store32(sm + F_MS, 128, 16384, R, hf * 4, st);
+            st32(sg + (size_t)(c + 1) * DD, st);
+        }
+        wait(2);
+        tload(p, trow + 192);
+        if (!krow && tr < L) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) p[i] += acc[i];
+            st32(yg + (size_t)(t0 + tr) * D, p);
+        }
+    }
+    if (wait.dead && (tid & 31) == 0) atomicExch(&g_mtc_timeout, 1);
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tmem_free_cols(tm, TCOLS);
+}
+
+// ───────────────────────────────── backward ────────────────────────────────
+constexpr int B_KQ = 0, B_YF = 49152, B_WZ = 98304, B_X = 147456, B_E = 196608;
+constexpr int B_TAB = B_E + 24576;
+constexpr int BWD_SMEM = B_TAB + (int)sizeof(Tables);
+
+// mstep: floats between the stored states of consecutive tile starts. SDER (exact rule on a full M
+// trajectory, no S stored): S at a tile start is M_t - (1 - alpha_{t-1}) M_{t-1}, and at the first token
+// (M_1 - r_0 M_0 + theta_0 e_0 k_0^T) / eta_0.
+template <int RULE, bool SOLVE, bool SDER>
+__global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int rd, long long mstep)
+{
+    constexpr bool HAS_S = (RULE == RULE_TITANS);
+    extern __shared__ __align__(1024) unsigned char sm[];
+    Tables& tb = *reinterpret_cast<Tables*>(sm + B_TAB);
+    float* Xb = reinterpret_cast<float*>(sm + B_WZ);                  // right-hand sides, fp32
+    float* Lb = reinterpret_cast<float*>(sm + B_WZ + TMAX * LDX * 4);     // Lx, fp32
+    float* Sd = reinterpret_cast<float*>(sm + B_X);                   // scan buffers X -> Xd, and Xs
+    float* Ss = reinterpret_cast<float*>(sm + B_X + 17408);
+    float* Gx = reinterpret_cast<float*>(sm + B_E);                   // G_M rows for the S rows
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int R = (warp & 3) * 32 + lane, hf = warp >> 2;
+    const int tr = R & 63;
+    const bool krow = R < 64;
+    const int b = blockIdx.x;
+    const size_t so = (size_t)b * a.seq_len * D + hf * 32, go = (size_t)b * a.seq_len;
+    const float* xg = (krow ? a.k : a.q) + so;
+    const float* yg = (krow ? a.v : a.d_y) + so;
+    const float* mtraj = a.m_traj + (size_t)b * a.traj_stride;
+    const float* straj = (HAS_S && !SDER) ? a.s_traj + (size_t)b * a.traj_stride : nullptr;
+    float* dxg = (krow ? a.d_k : a.d_q) + so;
+    const int n = a.t_end - a.t_start;
+    const int ntile = (n + T - 1) / T;
+
+    if (tid == 0) mbar_init(smem_u32(&tb.bar[0]), 1);
+    if (warp == 0) tmem_alloc_cols(reinterpret_cast<unsigned char*>(&tb.tmem), TCOLS);
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const unsigned tm = tb.tmem;
+    const unsigned trow = tm + ((unsigned)((warp & 3) * 32) << 16) + hf * 32;
+    Waiter wait{smem_u32(&tb.bar[0]), 0u, false};
+    const unsigned kq = smem_u32(sm + B_KQ), yf = smem_u32(sm + B_YF), wz = smem_u32(sm + B_WZ), xx = smem_u32(sm + B_X),
+                   ep = smem_u32(sm + B_E);
+    unsigned char* const kqp = sm + B_KQ;
+    unsigned char* const yfp = sm + B_YF;
+    unsigned char* const xxp = sm + B_X;
+
+    float g[32];                       // row of G_M (krow) or G_S, columns of this half
+    {
+        const float* seed = krow ? a.d_m_seed : a.d_s_seed;
+        ld32(g, seed + (size_t)b * DD + tr * D + hf * 32, (HAS_S || krow) && seed != nullptr);
+    }
+
+    for (int c = ntile - 1; c >= 0; c--) {
+        const int t0 = a.t_start + c * T, L = min(T, n - c * T);
+        const bool ok = tr < L;
+        auto state_row = [&](float (&x3)[32]) {      // this thread's row of M0 or S0
+            const float* mp = mtraj + (size_t)c * mstep;
+            if (krow) ld32(x3, mp + tr * D + hf * 32, true);
+            else if (HAS_S && !SDER) ld32(x3, straj + (size_t)c * mstep + tr * D + hf * 32, true);
+            else if (SDER) {
+                const float* m1 = (c > 0) ? mp : mp + DD;
+                const float* m0 = (c > 0) ? mp - DD : mp;
+                const int ta = (c > 0) ? t0 - 1 : t0;
+                const float r = 1.0f - a.alpha[go + ta];
+                float y3[32];
+                ld32(x3, m1 + tr * D + hf * 32, true);
+                ld32(y3, m0 + tr * D + hf * 32, true);
+#pragma unroll
+                for (int i = 0; i < 32; i++) x3[i] = fmaf(-r, y3[i], x3[i]);
+                if (c == 0) {
+                    const float* k0 = a.k + (so - hf * 32) + (size_t)t0 * D;
+                    float e = -a.v[(so - hf * 32) + (size_t)t0 * D + tr];
+                    for (int j = 0; j < D; j++) e = fmaf(m0[tr * D + j], k0[j], e);
+                    const float te = a.theta[go + t0] * e, et = a.eta[go + t0];
+                    const float inv = et > 1e-30f ? 1.0f / et : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 32; i++) x3[i] = fmaf(te, k0[hf * 32 + i], x3[i]) * inv;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) x3[i] = 0.f;
+            }
+        };
+        // ── stage 1: operands; K K^T | Q K^T and K,Q x M0,S0 ──
+        float y[32];                                 // V row (krow) or dY row
+        {
+            float x[32];
+            ld32(x, xg + (size_t)(t0 + tr) * D, ok);
+            ld32(y, yg + (size_t)(t0 + tr) * D, ok);
+            store32(kqp, 128, 16384, R, hf * 4, x);
+            if (!krow) store32(yfp, 128, 16384, R, hf * 4, y);
+        }
+        float dots[2];
+        {
+            float x3[32];
+            state_row(x3);
+            store32(xxp, 128, 16384, R, hf * 4, x3);
+            dots[0] = 0.f;
+#pragma unroll
+            for (int i = 0; i < 32; i++) dots[0] = fmaf(g[i], x3[i], dots[0]);     // <M0,G_M> or <S0,G_S>
+        }
+        if (tid < TMAX) {
+            const bool in = tid < L;
+            tb.gt[tid] = make_float4(in ? 1.0f - a.alpha[go + t0 + tid] : 1.f, (in && HAS_S) ? a.eta[go + t0 + tid] : 0.f,
+                                     in ? a.theta[go + t0 + tid] : 0.f, 0.f);
+        }
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<false, false>(tm, kq, 16384, 128, kq, 16384, 128, 64, 4);
+            mma6<false, false>(tm + 64, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        float w[32], p[32], au, bu;
+        const int u = krow ? (tr / rd) * rd - 1 : tr;
+        decay_row(tb.gt, u, hf, w, au, bu);
+        if (R == 64 + L - 1) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) tb.wM[hf * 32 + i] = w[i];
+            if (hf == 0) { tb.tot[0] = au; tb.tot[1] = bu; }
+        }
+        if (HAS_S && tid < TMAX) {
+            float hh = 1.f;
+            for (int i = L - 1; i > tid; i--) hh *= tb.gt[i].y;
+            tb.wS[tid] = (tid < L) ? tb.gt[tid].z * hh : 0.f;
+            if (tid == 0) tb.tot[2] = hh * tb.gt[0].y;
+        }
+        dots[1] = 0.f;
+        if (HAS_S && krow) {                          // <S0, G_M>
+#pragma unroll
+            for (int c8 = 0; c8 < 4; c8++) {
+                float s[8];
+                load8(s, xxp, 128, 16384, 64 + tr, hf * 4 + c8);
+#pragma unroll
+                for (int i = 0; i < 8; i++) dots[1] = fmaf(g[8 * c8 + i], s[i], dots[1]);
+            }
+        }
+        dots[0] = warp_sum(dots[0]); dots[1] = warp_sum(dots[1]);
+        if (lane == 0) { tb.red[warp][0] = dots[0]; tb.red[warp][1] = dots[1]; }
+        wait(0);
+        tload(p, trow);                               // k_t . k_j or q_t . k_j
+        {
+            float acc[32];
+            tload(acc, trow + 64);
+            if (krow) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) acc[i] = fmaf(au, acc[i], -y[i]);
+                if (HAS_S) {
+                    float s[32];
+                    tload(s, trow + 128);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) acc[i] = fmaf(bu, s[i], acc[i]);
+                }
+                st32(Xb + tr * LDX + hf * 32, acc);
+                if (SOLVE) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) acc[i] = w[i] * p[i];
+                    st32(Lb + tr * LDX + hf * 32, acc);
+                }
+            } else {
+                float zm = 0.f, zs = 0.f;
+#pragma unroll
+                for (int i = 0; i < 32; i++) zm = fmaf(y[i], acc[i], zm);
+                if (HAS_S) {
+                    tload(acc, trow + 128);
+#pragma unroll
+                    for (int i = 0; i < 32; i++) zs = fmaf(y[i], acc[i], zs);
+                }
+                tb.z[0][hf * 64 + tr] = zm; tb.z[1][hf * 64 + tr] = zs;
+            }
+        }
+        __syncthreads();
+        if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
+        // ── stage 2: E planes, W o P, G planes; right-hand side of F, E x G ──
+        {
+            const int row = tid & 63, q = tid >> 6;
+            float e[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
+                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
+            }
+            store8(sm + B_E, 64, 8192, row, 2 * q, e);
+            store8(sm + B_E, 64, 8192, row, 2 * q + 1, e + 8);
+        }
+        if (!krow) {
+            float wpv[32];
+#pragma unroll
+            for (int i = 0; i < 32; i++) wpv[i] = w[i] * p[i];
+            store32(sm + B_WZ + 24576, 64, 8192, tr, hf * 4, wpv);
+        }
+        store32(xxp, 128, 16384, R, hf * 4, g);
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<false, false>(tm, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);              // K G^T
+            mma6<true, true>(tm + 128, wz + 24576, 8192, 64, yf + 1024, 16384, 128, 64, 4);           // (W o P)^T dY
+            mma6<false, true>(tm + 192, ep, 8192, 64, xx, 16384, 128, 64, 4);                         // E G_M
+            if (HAS_S) mma6<false, true>(tm + 256, ep, 8192, 64, xx + 1024, 16384, 128, 64, 4);       // E G_S
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        float x3[32];
+        state_row(x3);
+        wait(0);
+        float dx[32];                                  // gradient of this thread's K or Q row
+        if (krow) {
+            const float wm = tb.wM[tr], wsv = HAS_S ? tb.wS[tr] : 0.f;
+            float s[32];
+            tload(dx, trow);
+            tload(s, trow + 128);
+#pragma unroll
+            for (int i = 0; i < 32; i++) dx[i] = -fmaf(wm, dx[i], s[i]);
+            if (HAS_S) {
+                tload(s, trow + 64);
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = fmaf(-wsv, s[i], dx[i]);
+            }
+            st32(Xb + tr * LDX + hf * 32, dx);
+            if (SOLVE) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) s[i] = w[i] * p[i];
+                st32(Lb + tr * LDX + hf * 32, s);
+            }
+            float gm = 0.f, gs = 0.f;
+            tload(s, trow + 192);
+#pragma unroll
+            for (int i = 0; i < 32; i++) dx[i] = -wm * s[i];
+#pragma unroll
+            for (int c8 = 0; c8 < 4; c8++) {
+                float kk[8];
+                load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
+#pragma unroll
+                for (int i = 0; i < 8; i++) gm = fmaf(kk[i], s[8 * c8 + i], gm);
+            }
+            if (HAS_S) {
+                tload(s, trow + 256);
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = fmaf(-wsv, s[i], dx[i]);
+#pragma unroll
+                for (int c8 = 0; c8 < 4; c8++) {
+                    float kk[8];
+                    load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) gs = fmaf(kk[i], s[8 * c8 + i], gs);
+                }
+            }
+            tb.z[2][hf * 64 + tr] = gm; tb.z[3][hf * 64 + tr] = gs;
+        }
+        __syncthreads();
+        if (SOLVE) solve_lower_t(Lb, Xb, (L + 15) >> 4);
+        // ── stage 3: F planes, dV, M0/S0 planes again; N | R, F and dY x M0,S0 ──
+        {
+            const int row = tid & 63, q = tid >> 6;
+            float e[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
+                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
+            }
+            store8(yfp, 128, 16384, row, 2 * q, e);
+            store8(yfp, 128, 16384, row, 2 * q + 1, e + 8);
+            if (row < L) {
+                float* dv = a.d_v + (so - hf * 32) + (size_t)(t0 + row) * D + 16 * q;
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    *reinterpret_cast<float4*>(dv + 4 * i) = make_float4(-e[4 * i], -e[4 * i + 1], -e[4 * i + 2], -e[4 * i + 3]);
+            }
+        }
+        store32(xxp, 128, 16384, R, hf * 4, x3);
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<false, false>(tm, yf, 16384, 128, ep, 8192, 64, 64, 4);                       // F,dY x E
+            mma6<false, true>(tm + 64, yf, 16384, 128, xx, 16384, 128, 64, 4);                 // F,dY x M0
+            if (HAS_S) mma6<false, true>(tm + 128, yf, 16384, 128, xx + 1024, 16384, 128, 64, 4);   // F,dY x S0
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        wait(0);
+        float zkm = 0.f, zks = 0.f;
+        {
+            float s[32];
+            tload(s, trow);                            // N row (krow) or R row
+#pragma unroll
+            for (int i = 0; i < 32; i++) { p[i] *= s[i]; s[i] *= -w[i]; }
+            store32(sm + B_WZ, 128, 16384, R, hf * 4, s);
+            if (!krow) {
+                // every read of the state planes by the tensor cores is over: the scan buffers take their place
+#pragma unroll
+                for (int i = 0; i < 32; i++) Sd[tr * LDS + hf * 32 + i] = p[i];
+                if (hf == 0) Sd[tr * LDS + 64] = tb.z[0][tr] + tb.z[0][64 + tr];
+                else Sd[tr * LDS + 65] = tb.z[1][tr] + tb.z[1][64 + tr];
+            }
+            tload(s, trow + 64);
+            if (krow) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = fmaf(au, s[i], dx[i]);
+                if (SOLVE) {
+#pragma unroll
+                    for (int c8 = 0; c8 < 4; c8++) {
+                        float kk[8];
+                        load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) zkm = fmaf(kk[i], s[8 * c8 + i], zkm);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = au * s[i];
+            }
+            if (HAS_S) {
+                tload(s, trow + 128);
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = fmaf(bu, s[i], dx[i]);
+                if (SOLVE && krow) {
+#pragma unroll
+                    for (int c8 = 0; c8 < 4; c8++) {
+                        float kk[8];
+                        load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) zks = fmaf(kk[i], s[8 * c8 + i], zks);
+                    }
+                }
+            }
+        }
+        publish();
+        // ── stage 4: (W o R, Z) x K and transposes; gate scans under them ──
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<false, true>(tm + 192, wz, 16384, 128, kq, 16384, 128, 64, 4);        // rows: Z K | -(W o R) K
+            mma6<true, true>(tm + 256, wz, 16384, 128, kq, 16384, 128, 64, 8);         // Z^T K - (W o R)^T Q
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        if (SOLVE) {
+            if (krow && u >= 0 && ok) {
+                if (rd == 1) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) Sd[u * LDS + hf * 32 + i] += p[i];
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) atomicAdd(&Sd[u * LDS + hf * 32 + i], p[i]);
+                }
+                atomicAdd(&Sd[u * LDS + 64], zkm);
+                if (HAS_S) atomicAdd(&Sd[u * LDS + 65], zks);
+            }
+            __syncthreads();
+        }
+        if (tid < 66) {                                // decayed scans, one column per thread
+            const int j = tid;
+            float sM, sS;
+            if (j < 64) { sM = tb.z[2][j] + tb.z[2][64 + j]; sS = tb.z[3][j] + tb.z[3][64 + j]; }
+            else {
+                sM = 0.f; sS = 0.f;
+#pragma unroll
+                for (int wq = 0; wq < 8; wq++) {
+                    const bool kw = (wq & 3) < 2;
+                    if (j == 64 && kw) sM += tb.red[wq][0];
+                    if (j == 65 && kw) sM += tb.red[wq][1];
+                    if (j == 65 && !kw) sS += tb.red[wq][0];
+                }
+            }
+            float xd = sM, xs = sS;
+            for (int s = L - 1; s >= 0; s--) {
+                const float4 gn = (s + 1 < L) ? tb.gt[s + 1] : make_float4(1.f, 1.f, 0.f, 0.f);
+                xd = fmaf(gn.x, xd, Sd[s * LDS + j]);
+                xs = fmaf(gn.y, xs, xd);
+                Sd[s * LDS + j] = xd;
+                Ss[s * LDS + j] = xs;
+            }
+            if (j < L) a.d_theta[go + t0 + j] = -Ss[j * LDS + j];
+        }
+        __syncthreads();
+        float s1 = 0.f, s2 = 0.f, hend = 1.f;
+        if (!krow) {
+            // row t + 1 of the decayed scans against row t of W and of theta_j h(j,t)
+            const float* xd = Sd + (tr + 1) * LDS + hf * 32;
+            const float* xs = Ss + (tr + 1) * LDS + hf * 32;
+            if (tr + 1 < L) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) s1 = fmaf(w[i], xd[i], s1);     // w is zero above the diagonal
+                if (HAS_S) {
+                    float hh = 1.f;
+                    for (int j = tr; j >= 0; j--) {
+                        if (j < tr) hh *= tb.gt[j + 1].y;
+                        if ((j >> 5) == hf) s2 = fmaf(tb.gt[j].z * hh, xs[j - hf * 32], s2);
+                    }
+                    hend = hh * tb.gt[0].y;
+                }
+            }
+            tb.part[0][hf * 64 + tr] = s1; tb.part[1][hf * 64 + tr] = s2;
+        }
+        // G_M rows for the S rows of the carry
+        if (krow && HAS_S) st32(Gx + tr * LDX + hf * 32, g);
+        __syncthreads();
+        if (!krow && hf == 0 && tr + 1 < L) {
+            const int t = tr + 1;
+            a.d_alpha[go + t0 + t] = -(fmaf(au, Sd[t * LDS + 64], bu * Sd[t * LDS + 65]) - (tb.part[0][tr] + tb.part[0][64 + tr]));
+            if (HAS_S) a.d_eta[go + t0 + t] = hend * Ss[t * LDS + 65] - (tb.part[1][tr] + tb.part[1][64 + tr]);
+        }
+        if (tid == 0) {
+            a.d_alpha[go + t0] = -Sd[64];
+            if (HAS_S) a.d_eta[go + t0] = Ss[65];
+        }
+        wait(0);
+        {
+            float s[32];
+            tload(s, trow + 192);
+#pragma unroll
+            for (int i = 0; i < 32; i++) dx[i] += s[i];
+            if (krow) {
+                tload(s, trow + 256);
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] += s[i];
+            }
+            if (ok) st32(dxg + (size_t)(t0 + tr) * D, dx);
+        }
+        __syncthreads();                               // the scan buffers have been read
+        // ── stage 5: carry. [diag(a) F ; diag(A) dY | diag(b) F ; diag(B) dY]^T [K ; Q] ──
+#pragma unroll
+        for (int c8 = 0; c8 < 4; c8++) {
+            float f[8], s[8];
+            load8(f, yfp, 128, 16384, R, hf * 4 + c8);
+#pragma unroll
+            for (int i = 0; i < 8; i++) s[i] = f[i] * au;
+            store8(sm + B_WZ, 128, 32768, R, hf * 4 + c8, s);
+            if (HAS_S) {
+#pragma unroll
+                for (int i = 0; i < 8; i++) s[i] = f[i] * bu;
+                store8(sm + B_WZ, 128, 32768, R, 8 + hf * 4 + c8, s);
+            }
+        }
+        publish();
+        if (tid == 0) {
+            fence_after_sync();
+            mma6<true, true>(tm + 320, wz, 32768, 128, kq, 16384, 128, 64, 8);
+            mma_commit(smem_u32(&tb.bar[0]));
+        }
+        const float At = tb.tot[0], Bt = tb.tot[1], Ht = tb.tot[2];
+        if (krow) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) g[i] *= At;
+        } else if (HAS_S) {
+            const float* gr = Gx + tr * LDX + hf * 32;
+#pragma unroll
+            for (int i = 0; i < 32; i++) g[i] = fmaf(Bt, gr[i], Ht * g[i]);
+        }
+        wait(0);
+        {
+            float s[32];
+            tload(s, trow + 320);
+            if (HAS_S || krow) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) g[i] += s[i];
+            }
+        }
+        fence_before_sync();
+        __syncthreads();
+    }
+
+    if ((HAS_S || krow) && a.d_m_out != nullptr) {
+        float* o = (krow ? a.d_m_out : a.d_s_out) + tr * D + hf * 32;
+        if (a.atomic_out) {
+#pragma unroll
+            for (int i = 0; i < 32; i++) atomicAdd(o + i, g[i]);
+        } else st32(o + (size_t)b * DD, g);
+    }
+    if (wait.dead && lane == 0) atomicExch(&g_mtc_timeout, 1);
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tmem_free_cols(tm, TCOLS);
+}
+
+}  // namespace mtc
+}  // namespace nlh

@@ -41,6 +41,8 @@ inline bool check_launch(const char* where) {
     return true;
 }
 
+inline bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
+
 enum Rule { RULE_DELTA = 0, RULE_TITANS = 1, RULE_HEBBIAN = 2 };
 
 // How the forward kernels emit memory states.
