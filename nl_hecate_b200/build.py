@@ -8,6 +8,7 @@ file so that it travels with the source tree.
 from __future__ import annotations
 
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -15,7 +16,6 @@ from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
-INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libnlh_b200.so")
 
@@ -33,13 +33,15 @@ def _nvcc() -> str:
     return nvcc
 
 
-def _deps(src: str):
-    yield os.path.join(CSRC, src)
-    for f in os.listdir(CSRC):
-        if f.endswith((".cuh", ".h")):
-            yield os.path.join(CSRC, f)
-    for f in os.listdir(INCLUDE):
-        yield os.path.join(INCLUDE, f)
+def _deps(path: str, seen=None):
+    """The file and everything it includes with quotes, recursively."""
+    seen = set() if seen is None else seen
+    path = os.path.normpath(path)
+    if path not in seen and os.path.exists(path):
+        seen.add(path)
+        for inc in re.findall(r'^\s*#include "([^"]+)"', open(path).read(), flags=re.M):
+            _deps(os.path.join(os.path.dirname(path), inc), seen)
+    return seen
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -50,7 +52,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     for s in srcs:
         obj = os.path.join(OBJ_DIR, s.replace(".cu", ".o"))
         objs.append(obj)
-        newest = max(os.path.getmtime(d) for d in _deps(s))
+        newest = max(os.path.getmtime(d) for d in _deps(os.path.join(CSRC, s)))
         if force or not os.path.exists(obj) or os.path.getmtime(obj) < newest:
             jobs.append([nvcc, *NVCC_FLAGS, "-c", os.path.join(CSRC, s), "-o", obj])
 

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
     Tables& tb = *reinterpret_cast<Tables*>(sm + F_TAB);
     float* Xb = reinterpret_cast<float*>(sm + F_X);      // right-hand side, then E, fp32
     float* Lb = reinterpret_cast<float*>(sm + F_E);      // Lx, fp32, until the solve is over
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = uniform_warp();
     const int R = (warp & 3) * 32 + (tid & 31), hf = warp >> 2;     // TMEM lane, column half
     const int tr = R & 63;                                          // token (or state row) of this thread
     const bool krow = R < 64;                                       // K / M rows, else Q / S rows
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
         store32(sm + F_KQ, 128, 16384, R, hf * 4, x);
         if (tid < TMAX) tb.gt[tid] = make_float4(1.0f - gal, get, gth, 0.f);
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, kq, 16384, 128, ms, 16384, 128, HAS_S ? 128 : 64, 4);     // K,Q x M0,S0
             mma6<false, false>(tm + 128, kq, 16384, 128, kq, 16384, 128, 64, 4);             // K,Q x K
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
             }
         }
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<true, true>(tm + 256, ew, 16384, 64, kq, 16384, 128, 64, 4);              // [Ew Es]^T K
             mma_commit(smem_u32(&tb.bar[1]));
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
     float* Sd = reinterpret_cast<float*>(sm + B_X);                   // scan buffers X -> Xd, and Xs
     float* Ss = reinterpret_cast<float*>(sm + B_X + 17408);
     float* Gx = reinterpret_cast<float*>(sm + B_E);                   // G_M rows for the S rows
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int R = (warp & 3) * 32 + lane, hf = warp >> 2;
     const int tr = R & 63;
     const bool krow = R < 64;
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                                      in ? a.theta[go + t0 + tid] : 0.f, 0.f);
         }
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, kq, 16384, 128, kq, 16384, 128, 64, 4);
             mma6<false, false>(tm + 64, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);
@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
         }
         store32(xxp, 128, 16384, R, hf * 4, g);
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);              // K G^T
             mma6<true, true>(tm + 128, wz + 24576, 8192, 64, yf + 1024, 16384, 128, 64, 4);           // (W o P)^T dY
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
         }
         store32(xxp, 128, 16384, R, hf * 4, x3);
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, yf, 16384, 128, ep, 8192, 64, 64, 4);                       // F,dY x E
             mma6<false, true>(tm + 64, yf, 16384, 128, xx, 16384, 128, 64, 4);                 // F,dY x M0
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
         }
         publish();
         // ── stage 4: (W o R, Z) x K and transposes; gate scans under them ──
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, true>(tm + 192, wz, 16384, 128, kq, 16384, 128, 64, 4);        // rows: Z K | -(W o R) K
             mma6<true, true>(tm + 256, wz, 16384, 128, kq, 16384, 128, 64, 8);         // Z^T K - (W o R)^T Q
@@ -926,7 +926,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
             }
         }
         publish();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<true, true>(tm + 320, wz, 32768, 128, kq, 16384, 128, 64, 8);
             mma_commit(smem_u32(&tb.bar[0]));

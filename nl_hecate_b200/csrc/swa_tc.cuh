@@ -134,9 +134,9 @@ __device__ int g_swa_tc_timeout = 0;   // set when a bounded mbarrier wait ran o
 //   E  softmax of tile i in registers (masks only on boundary tiles), P -> shared memory;
 //      O is rescaled in TMEM only by warps whose running maximum moved (tcgen05.ld/st)
 //   F  barrier; one thread issues O += P V(i)
-// TMA = true: Q, K and V tiles are staged by thread 0 with tiled TMA copies (see above) instead of
-// every thread's cp.async; only that thread waits for them (it is the one that issues the MMAs
-// that read them), on two alternating mbarriers with bounded waits.
+// TMA = true: Q, K and V tiles are staged by one thread of warp 0 with tiled TMA copies (see above)
+// instead of every thread's cp.async; only that warp waits for them (one of its threads issues the
+// MMAs that read them), on two alternating mbarriers with bounded waits.
 template <bool TMA>
 __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
     const __grid_constant__ CUtensorMap map_v)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = uniform_warp();
     const int qt = (gridDim.x - 1) - blockIdx.x;
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
     const size_t rs = (size_t)rs_in;                       // row stride of q, k, v (elements)
@@ -181,16 +181,16 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
         }
         return -1;
     };
-    // cp.async variant: every thread stages its part; TMA variant: thread 0 issues the copies onto
-    // the mbarrier ld_bar given by the caller
+    // cp.async variant: every thread stages its part; TMA variant: called by one elected thread, which
+    // issues the copies onto the mbarrier ld_bar given by the caller
     auto load_k = [&](int tile, int bufi, unsigned ld_bar) {
         const int k0 = tile * BN;
-        if (TMA) { if (tid == 0) tma_tile(smem_u32(smem + OFF_K + bufi * KV_BYTES), &map_k, h, k0, b, BN, ld_bar); }
+        if (TMA) { tma_tile(smem_u32(smem + OFF_K + bufi * KV_BYTES), &map_k, h, k0, b, BN, ld_bar); }
         else stage_rows(smem + OFF_K + bufi * KV_BYTES, k + base + (size_t)k0 * rs, rs, BN, min(BN, S - k0));
     };
     auto load_v = [&](int tile, int bufi, unsigned ld_bar) {
         const int k0 = tile * BN;
-        if (TMA) { if (tid == 0) tma_tile(smem_u32(smem + OFF_V + bufi * KV_BYTES), &map_v, h, k0, b, BN, ld_bar); }
+        if (TMA) { tma_tile(smem_u32(smem + OFF_V + bufi * KV_BYTES), &map_v, h, k0, b, BN, ld_bar); }
         else stage_rows(smem + OFF_V + bufi * KV_BYTES, v + base + (size_t)k0 * rs, rs, BN, min(BN, S - k0));
     };
     const unsigned idesc_qk = make_idesc(false), idesc_pv = make_idesc(true);
@@ -215,16 +215,17 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
     if (TMA) {
         // load group 0 on bar_ld: Q, K(0), V(0), K(1); group it+1 (issued in iteration it) goes to
         // bar_ld + 8 * ((it + 1) & 1) and is waited for by thread 0 in iteration it+1
-        if (tid == 0) {
-            const unsigned bytes = Q_BYTES + (kt >= 0 ? 2 * KV_BYTES : 0) + (nxt >= 0 ? KV_BYTES : 0);
-            mbar_expect_tx(bar_ld, bytes);
-            tma_tile(q_addr, &map_q, h, q0, b, BM, bar_ld);
-        }
-        if (kt >= 0) { load_k(kt, 0, bar_ld); load_v(kt, 0, bar_ld); }
-        if (nxt >= 0) load_k(nxt, 1, bar_ld);
-        if (tid == 0) {
+        if (warp == 0) {
+            if (elect_one()) {
+                const unsigned bytes = Q_BYTES + (kt >= 0 ? 2 * KV_BYTES : 0) + (nxt >= 0 ? KV_BYTES : 0);
+                mbar_expect_tx(bar_ld, bytes);
+                tma_tile(q_addr, &map_q, h, q0, b, BM, bar_ld);
+                if (kt >= 0) { load_k(kt, 0, bar_ld); load_v(kt, 0, bar_ld); }
+                if (nxt >= 0) load_k(nxt, 1, bar_ld);
+            }
             dead = !mbar_wait(bar_ld, 0, WAIT_LIMIT);
-            if (kt >= 0) { fence_after_sync(); issue_qk(0); }
+            __syncwarp();
+            if (kt >= 0 && elect_one()) { fence_after_sync(); issue_qk(0); }
         }
     } else {
         stage_rows(smem + OFF_Q, q + base + (size_t)q0 * rs, rs, BM, min(BM, S - q0));
@@ -235,7 +236,7 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
         fence_async_proxy();
         fence_before_sync();
         __syncthreads();
-        if (tid == 0 && kt >= 0) { fence_after_sync(); issue_qk(0); }
+        if (kt >= 0 && warp == 0 && elect_one()) { fence_after_sync(); issue_qk(0); }
     }
 
     float m_run = -INFINITY, l_run = 0.f;
@@ -262,12 +263,14 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
         // C: prefetch
         if (TMA) {
             const unsigned ld_next = bar_ld + 8 * ((it + 1) & 1);
-            if (tid == 0 && nxt >= 0) mbar_expect_tx(ld_next, (nxt2 >= 0 ? KV_BYTES : 0) + KV_BYTES);
-            if (nxt2 >= 0) load_k(nxt2, it & 1, ld_next);       // K(it+2) over K(it)
-            if (nxt >= 0) load_v(nxt, (it + 1) & 1, ld_next);   // V(it+1) over V(it-1)
-            // D: thread 0 waits for load group `it` (K(it+1), V(it)); the barrier is for the S
+            if (nxt >= 0 && warp == 0 && elect_one()) {
+                mbar_expect_tx(ld_next, (nxt2 >= 0 ? KV_BYTES : 0) + KV_BYTES);
+                if (nxt2 >= 0) load_k(nxt2, it & 1, ld_next);   // K(it+2) over K(it)
+                load_v(nxt, (it + 1) & 1, ld_next);             // V(it+1) over V(it-1)
+            }
+            // D: warp 0 waits for load group `it` (K(it+1), V(it)); the barrier is for the S
             // columns, which every thread has read by now
-            if (tid == 0 && it > 0 && !dead) dead = !mbar_wait(bar_ld + 8 * (it & 1), (unsigned)(it >> 1) & 1u, WAIT_LIMIT);
+            if (warp == 0 && it > 0 && !dead) dead = !mbar_wait(bar_ld + 8 * (it & 1), (unsigned)(it >> 1) & 1u, WAIT_LIMIT);
         } else {
             if (nxt2 >= 0) load_k(nxt2, it & 1, 0);            // K(it+2) over K(it)
             if (nxt >= 0) load_v(nxt, (it + 1) & 1, 0);        // V(it+1) over V(it-1)
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
         }
         fence_before_sync();
         __syncthreads();
-        if (tid == 0 && nxt >= 0) { fence_after_sync(); issue_qk((it + 1) & 1); }
+        if (nxt >= 0 && warp == 0 && elect_one()) { fence_after_sync(); issue_qk((it + 1) & 1); }
 
         // E: softmax
         const int k0 = kt * BN;
@@ -336,7 +339,7 @@ __global__ void __launch_bounds__(THREADS) swa_fwd_tc_kernel(
         fence_async_proxy();
         fence_before_sync();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             const unsigned v_addr = smem_u32(smem + OFF_V + (it & 1) * KV_BYTES);
 #pragma unroll

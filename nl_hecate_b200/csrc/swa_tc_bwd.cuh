@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dq_tc_kernel(
     TG* __restrict__ d_q, int S, int H, int window, int n_p, float scale, int rs_in, int rs_o)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int half = warp >> 2, row = (warp & 3) * 32 + lane;
     const int qt = (gridDim.x - 1) - blockIdx.x;
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dq_tc_kernel(
     fence_async_proxy();
     fence_before_sync();
     __syncthreads();
-    if (tid == 0 && kt >= 0) { fence_after_sync(); issue_scores(0); }
+    if (kt >= 0 && warp == 0 && elect_one()) { fence_after_sync(); issue_scores(0); }
 
     unsigned par_s = 0, par_o = 0;
     bool dead = false;
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dq_tc_kernel(
         fence_async_proxy();
         fence_before_sync();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             const unsigned k_addr = smem_u32(smem + DQ_OFF_K + (it & 1) * KV_BYTES);
 #pragma unroll
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dkv_tc_kernel(
     int rs_in, int rs_o)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int half = warp >> 2, row = (warp & 3) * 32 + lane;
     const int kt = blockIdx.x;
     const int bh = blockIdx.y, b = bh / H, h = bh - b * H;
@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dkv_tc_kernel(
     fence_async_proxy();
     fence_before_sync();
     __syncthreads();
-    if (tid == 0) { fence_after_sync(); issue_scores(0); }
+    if (warp == 0 && elect_one()) { fence_after_sync(); issue_scores(0); }
 
     const int kp = k0 + row;
     unsigned par_s = 0, par_o = 0;
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(BTHREADS, 2) swa_bwd_dkv_tc_kernel(
         fence_async_proxy();
         fence_before_sync();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after_sync();
             const unsigned q_addr = smem_u32(smem + KV_OFF_Q + bufi * KV_BYTES);
             const unsigned do_addr = smem_u32(smem + KV_OFF_DO + bufi * KV_BYTES);
