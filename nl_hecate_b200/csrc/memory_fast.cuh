@@ -1,4 +1,4 @@
-// Register-resident memory-rule kernels for head dimension D in {32, 64}.
+// Register-resident memory-rule kernels for head dimension D in {32, 64, 128}.
 //
 // One CTA per independent (batch x head) problem. The D x D memory M (and the
 // momentum S) never leave the register file during the sequence: D*D/16
@@ -90,12 +90,18 @@ struct ColReduce {
     }
     __device__ static __forceinline__ void run(const float2 (&v)[8], int lane, float (&out)[NOUT])
     {
-        static_assert(TPR == 4 || TPR == 2, "column reduction is written for 2 or 4 threads per row");
+        static_assert(TPR == 8 || TPR == 4 || TPR == 2, "column reduction is written for 2, 4 or 8 threads per row");
         float2 a4[4], a2[2];
 #pragma unroll
         for (int i = 0; i < 4; i++) a4[i] = add2(v[i], shfl_xor2(v[i + 4], 16));   // lane bit 4 <-> chunk bit 1
 #pragma unroll
         for (int i = 0; i < 2; i++) a2[i] = add2(a4[i], shfl_xor2(a4[i + 2], 8));  // lane bit 3 <-> chunk bit 0
+        if (TPR == 8) {           // lane bits 0-2 are columns: four consecutive sums per lane
+            out[0] = a2[0].x;
+            if (NOUT > 1) out[1 % NOUT] = a2[0].y;
+            if (NOUT > 2) { out[2 % NOUT] = a2[1].x; out[3 % NOUT] = a2[1].y; }
+            return;
+        }
         {   // lane bit 2 <-> pair within the chunk (not permuted: select)
             const bool up = lane & 4;
             const float2 send = up ? a2[0] : a2[1];
@@ -133,17 +139,17 @@ template <int D>
 constexpr size_t fast_fwd_smem_floats() { return (size_t)3 * 2 * FAST_TT * D + 2 * 3 * FAST_TT + FAST_TT * D; }
 // ring_mats: matrices per ring slot (2 when a stored S trajectory is read, else 1);
 // frozen: the per-chunk error buffer is only needed by the frozen rules.
-template <int D>
+template <int D, int SPLIT = 1>
 constexpr size_t fast_bwd_smem_floats(int ring_mats, bool frozen)
 {
-    using G = FastGeom<D>;
+    using G = FastGeom<D, SPLIT>;
     return (size_t)4 * 2 * FAST_TB * D        // k,v,q,dy tiles, double buffered
          + 2 * 3 * FAST_TB                    // gates
-         + (size_t)FAST_NST * ring_mats * D * D   // state ring
+         + (size_t)FAST_NST * ring_mats * G::ROWS * D   // state ring (this CTA's rows)
          + (size_t)2 * G::NW * FAST_TB * D    // dq / dk warp partials
-         + (size_t)FAST_TB * D                // dv staging
-         + (size_t)3 * FAST_TB * D            // per-row scalar partials
-         + (frozen ? (size_t)FAST_MAX_CHUNK * D : 0);   // errors of the current chunk
+         + (size_t)FAST_TB * G::ROWS          // dv staging
+         + (size_t)3 * FAST_TB * G::ROWS      // per-row scalar partials
+         + (frozen ? (size_t)FAST_MAX_CHUNK * G::ROWS : 0);   // errors of the current chunk
 }
 
 // xc: chunk permutation of the calling thread (0 = logical order).
@@ -437,11 +443,14 @@ __global__ void __launch_bounds__(FastGeom<D, SPLIT>::NT, (D == 64 && !FROZEN) ?
 // S_{t+1} = M_{t+1} - (1-alpha_t) M_t and S_{t+1} = eta_t S_t - theta_t e k^T,
 //   d_eta_t = <S_t, dS> = ( <M_{t+1} - (1-alpha_t) M_t, dS> + theta_t (e . dS k) ) / eta_t,
 // which needs eta_t > 0 (gates far below ~1e-3 lose accuracy to the division).
-template <int D, int RULE, bool FROZEN, bool SDER = false>
-__global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1) fast_bwd_kernel(BwdArgs a)
+// SPLIT > 1: the problem's rows are divided over SPLIT CTAs; each adds its partial column sums (d_q,
+// d_k) and gate gradients with atomicAdd into outputs that the launcher has zeroed.
+template <int D, int RULE, bool FROZEN, bool SDER = false, int SPLIT = 1>
+__global__ void __launch_bounds__(FastGeom<D, SPLIT>::NT, (D == 64 && !FROZEN) ? 2 : 1) fast_bwd_kernel(BwdArgs a)
 {
-    using G = FastGeom<D>;
-    constexpr int NT = G::NT, TPR = G::TPR, NW = G::NW, TB = FAST_TB, NST = FAST_NST;
+    using G = FastGeom<D, SPLIT>;
+    constexpr int ROWS = G::ROWS;
+    constexpr int NT = G::NT, TPR = G::TPR, NW = G::NW, TB = FAST_TB, NST = FAST_NST, SD = ROWS * D;
     constexpr int NOUT = ColReduce<TPR>::NOUT;
     extern __shared__ __align__(16) float sm[];
     float* kt = sm;                                   // [2][TB][D]
@@ -450,17 +459,19 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
     float* dyt = qt + 2 * TB * D;
     float* gt = dyt + 2 * TB * D;                     // [2][3][TB]
     constexpr int RM = (RULE == RULE_TITANS && !SDER) ? 2 : 1;   // matrices per ring slot
-    float* ring = gt + 2 * 3 * TB;                    // [NST][RM][D*D]
-    float* pq = ring + (size_t)NST * RM * D * D;      // [NW][TB][D]
+    float* ring = gt + 2 * 3 * TB;                    // [NST][RM][ROWS*D]
+    float* pq = ring + (size_t)NST * RM * SD;      // [NW][TB][D]
     float* pk = pq + (size_t)NW * TB * D;             // [NW][TB][D]
-    float* dvs = pk + (size_t)NW * TB * D;            // [TB][D]
-    float* scp = dvs + TB * D;                        // [3][TB][D] per-row partials
-    float* es = scp + 3 * TB * D;                     // [FAST_MAX_CHUNK][D], frozen rules only
+    float* dvs = pk + (size_t)NW * TB * D;            // [TB][ROWS]
+    float* scp = dvs + TB * ROWS;                     // [3][TB][ROWS] per-row partials
+    float* es = scp + 3 * TB * ROWS;                  // [FAST_MAX_CHUNK][ROWS], frozen rules only
 
-    const int tid = threadIdx.x, r = tid / TPR, cg = tid % TPR;
+    const int tid = threadIdx.x, cg = tid % TPR;
+    const int part = (SPLIT > 1) ? (int)(blockIdx.x % SPLIT) : 0;
+    const int rl = tid / TPR, r = part * ROWS + rl;      // row within the CTA, row of the state
     const int lane = tid & 31, warp = tid >> 5;
     const size_t dd = (size_t)D * D;
-    const int b = blockIdx.x;
+    const int b = blockIdx.x / SPLIT;
     const size_t so = (size_t)b * a.seq_len * D, go = (size_t)b * a.seq_len;
     const float* k = a.k + so; const float* v = a.v + so; const float* q = a.q + so;
     const float* dy = a.d_y + so;
@@ -526,7 +537,7 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                     float e;
                     if (FROZEN) e = fast_fwd_token<D, RULE>(Mc, Sc, M0, kt + tl * D, vt[tl * D + r], al, th, et, cg, xc);
                     else e = fast_fwd_token<D, RULE>(Mc, Sc, Mc, kt + tl * D, vt[tl * D + r], al, th, et, cg, xc);
-                    if (FROZEN && cg == 0) es[(t - t0) * D + r] = e;
+                    if (FROZEN && cg == 0) es[(t - t0) * ROWS + rl] = e;
                     store_state8<D>(Mc, mrec + (size_t)(t - t0 + 1) * dd, r, cg, xc);
                     if (RULE == RULE_TITANS) store_state8<D>(Sc, srec + (size_t)(t - t0 + 1) * dd, r, cg, xc);
                 }
@@ -568,11 +579,11 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
         const ptrdiff_t sdiff = (RULE == RULE_TITANS && !SDER) ? (st_base - mt_base) : 0;
         auto prefetch_state = [&]() {
             if (jp >= 0) {
-                float* dst = ring_t + pslot * (RM * DD);
+                float* dst = ring_t + pslot * (RM * SD);
 #pragma unroll
                 for (int jj = 0; jj < 4; jj++) {
                     cp_async16(dst + jj * NT * 4, gpre + co[jj]);
-                    if (RULE == RULE_TITANS && !SDER) cp_async16(dst + DD + jj * NT * 4, gpre + sdiff + co[jj]);
+                    if (RULE == RULE_TITANS && !SDER) cp_async16(dst + SD + jj * NT * 4, gpre + sdiff + co[jj]);
                 }
             }
             jp--;
@@ -604,7 +615,7 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                 if (tl == ntok - 1 && tile < ntl - 1 && (t1 - (tt0 + TB)) < NST) cp_async_wait<0>();
                 else cp_async_wait<NST - 1>();
                 if (tl == ntok - 1) __syncthreads();   // tile streams (other threads' copies) visible
-                const float* ms = ring_t + cslot * (RM * DD);
+                const float* ms = ring_t + cslot * (RM * SD);
                 cslot = (cslot == 0) ? NST - 1 : cslot - 1;
                 float2 Mt[8], St[8], kk[8], qq[8];
 #pragma unroll
@@ -612,7 +623,7 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                     const float4 t4 = *reinterpret_cast<const float4*>(ms + jj * NT * 4);
                     Mt[2 * jj] = make_float2(t4.x, t4.y); Mt[2 * jj + 1] = make_float2(t4.z, t4.w);
                     if (RULE == RULE_TITANS && !SDER) {
-                        const float4 s4 = *reinterpret_cast<const float4*>(ms + DD + jj * NT * 4);
+                        const float4 s4 = *reinterpret_cast<const float4*>(ms + SD + jj * NT * 4);
                         St[2 * jj] = make_float2(s4.x, s4.y); St[2 * jj + 1] = make_float2(s4.z, s4.w);
                     }
                 }
@@ -655,7 +666,7 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                 const float u = row_allreduce<TPR>(us.x + us.y);
                 float e = 0.f;
                 if (RULE != RULE_HEBBIAN) {
-                    if (FROZEN) e = es[j * D + r];
+                    if (FROZEN) e = es[j * ROWS + rl];
                     else e = row_allreduce<TPR>(p2.x + p2.y) - vr;
                 }
                 const float de = -th * u;
@@ -664,11 +675,11 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                 float pe = 0.f;
                 if (RULE == RULE_TITANS) pe = row_allreduce<TPR>(pe2.x + pe2.y);
                 if (cg == 0) {
-                    scp[(0 * TB + tl) * D + r] = pa;
-                    scp[(1 * TB + tl) * D + r] = (RULE != RULE_HEBBIAN) ? e * u : 0.f;
+                    scp[(0 * TB + tl) * ROWS + rl] = pa;
+                    scp[(1 * TB + tl) * ROWS + rl] = (RULE != RULE_HEBBIAN) ? e * u : 0.f;
                     if (SDER) pe = (et > 1e-30f) ? __fdividef(pe + th * e * u, et) : 0.f;
-                    scp[(2 * TB + tl) * D + r] = pe;
-                    dvs[tl * D + r] = (RULE == RULE_HEBBIAN) ? u : th * u;
+                    scp[(2 * TB + tl) * ROWS + rl] = pe;
+                    dvs[tl * ROWS + rl] = (RULE == RULE_HEBBIAN) ? u : th * u;
                 }
 
                 // pass 2: column partials d_q = M_{t+1}^T dy ; d_k = -theta G^T e + Mk^T de
@@ -705,20 +716,30 @@ __global__ void __launch_bounds__(FastGeom<D>::NT, (D == 64 && !FROZEN) ? 2 : 1)
                 float sq = 0.f, sk = 0.f;
 #pragma unroll
                 for (int w = 0; w < NW; w++) { sq += pq[(size_t)w * TB * D + i]; sk += pk[(size_t)w * TB * D + i]; }
-                dq[(size_t)tt0 * D + i] = sq;
-                dk[(size_t)tt0 * D + i] = sk;
-                dv[(size_t)tt0 * D + i] = dvs[i];
+                if (SPLIT > 1) {
+                    atomicAdd(dq + (size_t)tt0 * D + i, sq);
+                    atomicAdd(dk + (size_t)tt0 * D + i, sk);
+                } else {
+                    dq[(size_t)tt0 * D + i] = sq;
+                    dk[(size_t)tt0 * D + i] = sk;
+                    dv[(size_t)tt0 * D + i] = dvs[i];
+                }
             }
+            if (SPLIT > 1)
+                for (int i = tid; i < ntok * ROWS; i += NT) {
+                    const int tl = i / ROWS, c2 = i - tl * ROWS;
+                    dv[(size_t)(tt0 + tl) * D + part * ROWS + c2] = dvs[i];
+                }
             for (int job = warp; job < 3 * ntok; job += NW) {
                 const int which = job / ntok, tl = job - which * ntok;
                 if ((which == 1 && RULE == RULE_HEBBIAN) || (which == 2 && RULE != RULE_TITANS)) continue;
                 float s = 0.f;
-                for (int i = lane; i < D; i += 32) s += scp[(which * TB + tl) * D + i];
+                for (int i = lane; i < ROWS; i += 32) s += scp[(which * TB + tl) * ROWS + i];
                 s = warp_sum(s);
                 if (lane == 0) {
-                    if (which == 0) dalpha[tt0 + tl] = -s;
-                    else if (which == 1) dtheta[tt0 + tl] = -s;
-                    else deta[tt0 + tl] = s;
+                    float* dst = which == 0 ? dalpha + tt0 + tl : which == 1 ? dtheta + tt0 + tl : deta + tt0 + tl;
+                    const float val = which == 2 ? s : -s;
+                    if (SPLIT > 1) atomicAdd(dst, val); else *dst = val;
                 }
             }
             // the next tile's first-token barrier orders these reads before pq/pk/scp are rewritten
@@ -751,6 +772,9 @@ inline bool fast_common_ok(int d, float clip, float mmax)
 {
     return (d == 64 || d == 32) && !(clip > 0.0f) && !m_norm_enabled(mmax);
 }
+// D = 128 (8 threads per row): one problem's state is 64 KB per matrix, so its rows are always divided
+// over CTAs; the launches below exist with both trajectories stored (or M for Delta / Hebbian).
+inline bool fast_128_ok(int d, float clip, float mmax) { return d == 128 && !(clip > 0.0f) && !m_norm_enabled(mmax); }
 
 // Number of SMs of the current device (queried once per process).
 inline int sm_count()
@@ -770,6 +794,31 @@ inline int sm_count()
 // problems of 512 tokens: forward 0.27 -> 0.19 ms, M-only backward 0.48 -> 0.42 ms; with 128
 // problems two CTAs would share an SM and nothing is gained).
 inline bool split_rows(int d, int batch) { return d == 64 && 2 * batch <= sm_count() && option_value(NLH_OPT_ROW_SPLIT) != 0; }
+
+// Rows of a D = 128 problem per CTA: 16 while all CTAs then still find room at once (two per SM), else
+// 32. The kernels are bound by the token chain of a CTA when few CTAs run, by the k/v/q streams that
+// every CTA of a problem reads again when many do.
+inline bool split_128_fine(int batch) { return batch * 8 <= 2 * sm_count(); }
+
+template <int RULE, bool FROZEN, int SPLIT>
+static void fwd128_launch(const FwdArgs& a, cudaStream_t st)
+{
+    const size_t smem = fast_fwd_smem_floats<128>() * sizeof(float);
+    cudaFuncSetAttribute(fast_fwd_kernel<128, RULE, FROZEN, SPLIT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    fast_fwd_kernel<128, RULE, FROZEN, SPLIT, true><<<a.batch * SPLIT, FastGeom<128, SPLIT>::NT, smem, st>>>(a);
+}
+template <int RULE>
+static bool fast_fwd_launch_128(const FwdArgs& a, cudaStream_t st)
+{
+    if constexpr (RULE != RULE_HEBBIAN) {
+        if (a.frozen) {
+            if (split_128_fine(a.batch)) fwd128_launch<RULE, true, 8>(a, st); else fwd128_launch<RULE, true, 4>(a, st);
+            return true;
+        }
+    }
+    if (split_128_fine(a.batch)) fwd128_launch<RULE, false, 8>(a, st); else fwd128_launch<RULE, false, 4>(a, st);
+    return true;
+}
 
 template <int D, int RULE>
 static bool fast_fwd_launch(const FwdArgs& a, cudaStream_t st)
@@ -807,14 +856,22 @@ static bool fast_fwd_launch(const FwdArgs& a, cudaStream_t st)
 // Returns true when a fast kernel was launched (caller checks the launch).
 static bool fast_forward(int rule, const FwdArgs& a, cudaStream_t st)
 {
-    if (!fast_common_ok(a.d, a.error_clip, a.m_norm_max)) return false;
+    const bool wide = fast_128_ok(a.d, a.error_clip, a.m_norm_max);
+    if (!wide && !fast_common_ok(a.d, a.error_clip, a.m_norm_max)) return false;
     if (a.frozen && rule == RULE_HEBBIAN) return false;
+    if (wide && rule == RULE_TITANS && a.s_out == nullptr) return false;
     const bool al = aligned16(a.k) && aligned16(a.v) && aligned16(a.q) && aligned16(a.y) &&
                     aligned16(a.m_init) && aligned16(a.m_out) &&
                     (rule != RULE_TITANS || (aligned16(a.s_init) && aligned16(a.s_out))) &&
                     (a.s_out != nullptr || rule != RULE_TITANS || a.store_mode == STORE_ALL) &&
                     (a.init_stride % 4 == 0) && (a.out_stride % 4 == 0);
     if (!al) return false;
+    if (wide) {
+        if (rule == RULE_TITANS) return fast_fwd_launch_128<RULE_TITANS>(a, st);
+        if (rule == RULE_DELTA) return fast_fwd_launch_128<RULE_DELTA>(a, st);
+        if (rule == RULE_HEBBIAN) return fast_fwd_launch_128<RULE_HEBBIAN>(a, st);
+        return false;
+    }
     if (a.d == 64) {
         if (rule == RULE_TITANS) return fast_fwd_launch<64, RULE_TITANS>(a, st);
         if (rule == RULE_DELTA) return fast_fwd_launch<64, RULE_DELTA>(a, st);
@@ -847,9 +904,39 @@ static bool fast_bwd_launch(const BwdArgs& a, cudaStream_t st)
     return true;
 }
 
+template <int RULE, bool FROZEN, int SPLIT>
+static void bwd128_launch(const BwdArgs& a, cudaStream_t st)
+{
+    const size_t smem = fast_bwd_smem_floats<128, SPLIT>(RULE == RULE_TITANS ? 2 : 1, FROZEN) * sizeof(float);
+    cudaFuncSetAttribute(fast_bwd_kernel<128, RULE, FROZEN, false, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    fast_bwd_kernel<128, RULE, FROZEN, false, SPLIT><<<a.batch * SPLIT, FastGeom<128, SPLIT>::NT, smem, st>>>(a);
+}
+template <int RULE>
+static bool fast_bwd_launch_128(const BwdArgs& a, cudaStream_t st)
+{
+    // the CTAs of a problem add into d_q, d_k and the gate gradients: zero the token range they cover
+    const int t0 = a.chunk > 0 ? 0 : a.t_start, n = (a.chunk > 0 ? a.seq_len : a.t_end) - t0;
+    auto zero = [&](float* p, int w) {
+        if (p != nullptr) cudaMemset2DAsync(p + (size_t)t0 * w, (size_t)a.seq_len * w * 4, 0, (size_t)n * w * 4, a.batch, st);
+    };
+    zero(a.d_q, 128); zero(a.d_k, 128); zero(a.d_alpha, 1);
+    if (RULE != RULE_HEBBIAN) zero(a.d_theta, 1);
+    if (RULE == RULE_TITANS) zero(a.d_eta, 1);
+    if constexpr (RULE != RULE_HEBBIAN) {
+        if (a.frozen) {
+            if (split_128_fine(a.batch)) bwd128_launch<RULE, true, 8>(a, st); else bwd128_launch<RULE, true, 4>(a, st);
+            return true;
+        }
+    }
+    if (split_128_fine(a.batch)) bwd128_launch<RULE, false, 8>(a, st); else bwd128_launch<RULE, false, 4>(a, st);
+    return true;
+}
+
 static bool fast_backward(int rule, BwdArgs& a, cudaStream_t st)
 {
-    if (!fast_common_ok(a.d, a.error_clip, a.m_norm_max)) return false;
+    const bool wide = fast_128_ok(a.d, a.error_clip, a.m_norm_max);
+    if (!wide && !fast_common_ok(a.d, a.error_clip, a.m_norm_max)) return false;
+    if (wide && rule == RULE_TITANS && a.s_traj == nullptr) return false;
     if (a.frozen && (rule == RULE_HEBBIAN || a.chunk > FAST_MAX_CHUNK)) return false;
     if (a.t_end <= a.t_start && a.chunk <= 0) return false;
     const bool al = aligned16(a.k) && aligned16(a.v) && aligned16(a.q) && aligned16(a.d_y) &&
@@ -867,6 +954,12 @@ static bool fast_backward(int rule, BwdArgs& a, cudaStream_t st)
         if (!ws) return false;
         a.m_rec = (float*)ws;
         a.s_rec = (float*)(ws + per);
+    }
+    if (wide) {
+        if (rule == RULE_TITANS) return fast_bwd_launch_128<RULE_TITANS>(a, st);
+        if (rule == RULE_DELTA) return fast_bwd_launch_128<RULE_DELTA>(a, st);
+        if (rule == RULE_HEBBIAN) return fast_bwd_launch_128<RULE_HEBBIAN>(a, st);
+        return false;
     }
     if (a.d == 64) {
         if (rule == RULE_TITANS) return fast_bwd_launch<64, RULE_TITANS>(a, st);
