@@ -67,7 +67,7 @@ static int run_forward(int rule, FwdArgs a, const char* where)
         return NLH_ERR_INVALID_ARG;
     }
     cudaStream_t st = current_stream();
-    if (option_value(NLH_OPT_CHUNK_MATRIX) && mtc::forward(rule, a, a.frozen ? a.interval : 1, st))
+    if (option_value(NLH_OPT_CHUNK_MATRIX) && mtc::forward(rule, a, st))
         return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (fast_forward(rule, a, st)) return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (rule == RULE_TITANS && a.s_out == nullptr) {
@@ -98,8 +98,8 @@ static int run_forward(int rule, FwdArgs a, const char* where)
 static bool tile_backward(int rule, const BwdArgs& a, cudaStream_t st)
 {
     const long long dd = (long long)a.d * a.d;
-    if (a.chunk > 0) return mtc::backward(rule, a, a.chunk, a.frozen ? a.chunk : 1, dd, st);
-    return !a.frozen && a.t_end - a.t_start >= 24 && mtc::backward(rule, a, 64, 1, 64 * dd, st);
+    if (a.chunk > 0) return mtc::backward(rule, a, a.chunk, dd, st);
+    return !a.frozen && a.t_end - a.t_start >= 24 && mtc::backward(rule, a, 64, 64 * dd, st);
 }
 
 static int run_backward(int rule, BwdArgs a, const char* where)

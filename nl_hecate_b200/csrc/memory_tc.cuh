@@ -1,5 +1,5 @@
 // Titans / Delta memory rule in CHUNK-PARALLEL (matrix) form on the 5th-generation tensor cores,
-// head dimension 64: exact rule, frozen-M0 rule, and frozen rule with several chunks per tile.
+// head dimension 64: exact rule, and frozen-M0 rule with one chunk per tile.
 //
 // A problem's tokens are cut into tiles of up to 64. Inside a tile everything is linear in the
 // tile-start state (M0, S0) and the errors E (rows e_t). With r_t = 1 - alpha_t and, for t >= j,
@@ -8,8 +8,8 @@
 //     A_t = prod_{i<=t} r_i,  H_t = prod_{i<=t} eta_i,  B_t = eta_0 Om(t,0)   (weights of M0, S0)
 //     W(t,j) = theta_j Om(t,j)
 // the state after token t is  M_t = A_t M0 + B_t S0 - sum_{j<=t} W(t,j) e_j k_j^T. The error of
-// token t is read from the state of index u(t): t-1 for the exact rule, the last token before its
-// chunk for the frozen rule (u = -1: the tile-start state). With a_t = A_u, b_t = B_u (1, 0 for u = -1)
+// token t is read from the state of index u(t): t-1 for the exact rule, -1 (the tile-start state) for
+// the frozen rule. With a_t = A_u, b_t = B_u (1, 0 for u = -1)
 //     (I + Lx) E = diag(a) K M0^T + diag(b) K S0^T - V ,   Lx(t,j) = W(u(t),j) (k_t . k_j)
 //     Y   = diag(A) Q M0^T + diag(B) Q S0^T - (W o P) E ,  P = Q K^T
 //     M_C = A_L M0 + B_L S0 - E^T diag(W(L-1,:)) K ,       S_C = H_L S0 - E^T diag(theta_j h(j,L-1)) K
@@ -137,6 +137,7 @@ struct Tables {
     float4 gt[TMAX];            // r_t, eta_t, theta_t of the tile's tokens (padding: 1, 0, 0)
     float wM[TMAX], wS[TMAX];   // W(L-1,j), theta_j h(j,L-1)
     float tot[8];               // A_L, B_L, H_L
+    float2 ab[TMAX];            // A_t, B_t
     float z[4][2 * TMAX];       // backward: row dots of the two column halves (zM, zS, gm, gs)
     float part[2][2 * TMAX];
     float red[8][4];
@@ -144,28 +145,49 @@ struct Tables {
     unsigned tmem;
 };
 
-// Row u of W for this thread's 32 columns (half hf): w[i] = W(u, 32 hf + i), and A_u, B_u.
-__device__ __forceinline__ void decay_row(const float4* gt, int u, int hf, float (&w)[32], float& au, float& bu)
+// W of the tile as a table [TMAX][LDX], row t: W(t, j), zero above the diagonal; tb.ab[t] = A_t, B_t;
+// tb.wS[j] = theta_j h(j, L-1); tb.tot = A_L, B_L, H_L; tb.wM = W(L-1, .). One thread per column j, the
+// recurrence runs over t: h' = eta_t h, Om' = r_t Om + h'. (One row per thread, unrolled, was 500
+// instructions that every warp fetched once per tile: 2.5k cycles against 1k here.)
+template <bool HAS_S>
+__device__ __forceinline__ void decay_table(Tables& tb, float* Wt, int tid, int L)
 {
-    float rho = 1.f, om = 1.f;
-    auto step = [&](int j) {       // from column j+1 to column j
-        const float4 g = gt[j + 1];
-        const bool in = j < u;
-        rho = in ? rho * g.x : 1.f;
-        om = in ? fmaf(g.y, om, rho) : 1.f;
-    };
-    w[31] = (63 <= u) ? gt[63].z : 0.f;
-#pragma unroll
-    for (int j = 62; j >= 32; j--) { step(j); w[j - 32] = (j <= u) ? gt[j].z * om : 0.f; }
-    if (hf == 0) {
-#pragma unroll
-        for (int j = 31; j >= 0; j--) { step(j); w[j] = (j <= u) ? gt[j].z * om : 0.f; }
-    } else {
-#pragma unroll
-        for (int j = 31; j >= 0; j--) step(j);
+    if (tid >= 0 && tid < TMAX) {
+        const int j = tid;
+        const float th = tb.gt[j].z;
+        float om = 0.f, h = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < TMAX; t++) {
+            const float4 g = tb.gt[t];
+            h = t == j ? 1.f : g.y * h;
+            om = fmaf(g.x, om, h);
+            if (!HAS_S) om = t == j ? 1.f : om;
+            Wt[t * LDX + j] = th * om;
+            if (t == L - 1) { tb.wM[j] = th * om; if (HAS_S) tb.wS[j] = th * h; }
+        }
+    } else if (tid == TMAX) {
+        float aa = 1.f, h = 1.f, om = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < TMAX; t++) {
+            const float4 g = tb.gt[t];
+            aa *= g.x; h *= g.y; om = fmaf(g.x, om, h);
+            tb.ab[t] = make_float2(aa, HAS_S ? om : 0.f);
+            if (t == L - 1) { tb.tot[0] = aa; tb.tot[1] = HAS_S ? om : 0.f; tb.tot[2] = h; }
+        }
     }
-    au = (u >= 0) ? rho * gt[0].x : 1.f;
-    bu = (u >= 0) ? om * gt[0].y : 0.f;
+}
+// Row u of the table for this thread's 32 columns (half hf), and A_u, B_u; u = -1: no token before
+__device__ __forceinline__ void decay_row(const Tables& tb, const float* Wt, int u, int hf, float (&w)[32], float& au, float& bu)
+{
+    const float* row = Wt + max(u, 0) * LDX + hf * 32;
+    const float2 ab = tb.ab[max(u, 0)];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const float4 x = *reinterpret_cast<const float4*>(row + 4 * i);
+        w[4 * i] = u < 0 ? 0.f : x.x; w[4 * i + 1] = u < 0 ? 0.f : x.y; w[4 * i + 2] = u < 0 ? 0.f : x.z; w[4 * i + 3] = u < 0 ? 0.f : x.w;
+    }
+    au = u < 0 ? 1.f : ab.x;
+    bu = u < 0 ? 0.f : ab.y;
 }
 
 // X <- (I + Lo)^{-1} X and X <- (I + Lo)^{-T} X for the strictly lower triangular Lo [n16*16 rows],
@@ -179,16 +201,19 @@ __device__ __forceinline__ void diag16(const float* __restrict__ Lo, float* X, i
 #pragma unroll
     for (int i = 1; i < 16; i++) {
         const float* row = Lo + (r0 + i) * LDX + r0;
+        float s[4] = {0.f, 0.f, 0.f, 0.f};            // four sums: only the last term waits for row i - 1
 #pragma unroll
         for (int j4 = 0; j4 < i; j4 += 4) {
             const float4 l = *reinterpret_cast<const float4*>(row + j4);
-            x[i] = fmaf(-l.x, x[j4], x[i]);
-            if (j4 + 1 < i) x[i] = fmaf(-l.y, x[j4 + 1], x[i]);
-            if (j4 + 2 < i) x[i] = fmaf(-l.z, x[j4 + 2], x[i]);
-            if (j4 + 3 < i) x[i] = fmaf(-l.w, x[j4 + 3], x[i]);
+            s[0] = fmaf(l.x, x[j4], s[0]);
+            if (j4 + 1 < i) s[1] = fmaf(l.y, x[j4 + 1], s[1]);
+            if (j4 + 2 < i) s[2] = fmaf(l.z, x[j4 + 2], s[2]);
+            if (j4 + 3 < i) s[3] = fmaf(l.w, x[j4 + 3], s[3]);
         }
-        X[(r0 + i) * LDX + c] = x[i];
+        x[i] -= (s[0] + s[1]) + (s[2] + s[3]);
     }
+#pragma unroll
+    for (int i = 1; i < 16; i++) X[(r0 + i) * LDX + c] = x[i];
 }
 __device__ __forceinline__ void diag16_t(const float* __restrict__ Lo, float* X, int r0, int c)
 {
@@ -283,6 +308,45 @@ __device__ __forceinline__ void st32(float* p, const float (&v)[32])
     for (int i = 0; i < 8; i++)
         *reinterpret_cast<float4*>(p + 4 * i) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
 }
+// Global memory is read and written in units of 8 rows x 32 columns per warp (a lane: 8 columns of one
+// row): 8 lines of 128 bytes per instruction, where one row per lane touches 32. Unit i of a warp:
+// rows 32 i + 8 (warp / 2) .. + 7, columns 32 (warp % 2) .. + 31; 64 rows are units 0 and 1.
+struct Unit {
+    int row0, cc;              // row of unit 0; 8-column chunk
+    __device__ __forceinline__ Unit(int warp, int lane) : row0((warp >> 1) * 8 + (lane & 7)), cc((warp & 1) * 4 + (lane >> 3)) {}
+    __device__ __forceinline__ int row(int i) const { return row0 + 32 * i; }
+};
+__device__ __forceinline__ void ld8(float* v, const float* __restrict__ p)
+{
+    const float4 x = *reinterpret_cast<const float4*>(p), y = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+}
+// rows past the tile's L tokens: row 0 is read and dropped, so that every load is in flight at once
+__device__ __forceinline__ void ld8_row(float* v, const float* __restrict__ tile, int r, int L)
+{
+    ld8(v, tile + (r < L ? r : 0) * D);
+}
+__device__ __forceinline__ void zero_past(float* v, int r, int L)
+{
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = r < L ? v[j] : 0.f;
+}
+__device__ __forceinline__ void st8(float* p, const float* v)
+{
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
+}
+// 8 columns of one row of a staged matrix to global memory
+__device__ __forceinline__ void copy8(float* g, const float* s)
+{
+    const float4 x = *reinterpret_cast<const float4*>(s), y = *reinterpret_cast<const float4*>(s + 4);
+    *reinterpret_cast<float4*>(g) = x; *reinterpret_cast<float4*>(g + 4) = y;
+}
+// asks for `bytes` (a multiple of 16) of global memory to be brought into L2
+__device__ __forceinline__ void l2_prefetch(const float* p, unsigned bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tload(float (&v)[32], unsigned taddr)
 {
     unsigned r[32];
@@ -317,10 +381,10 @@ constexpr int F_KQ = 0, F_MS = 49152, F_WP = 98304, F_E = 122880, F_EW = 147456,
 constexpr int F_TAB = F_X + TMAX * LDX * 4;
 constexpr int FWD_SMEM = F_TAB + (int)sizeof(Tables);
 
-// T tokens per tile; rd tokens per frozen chunk (1: exact rule, T: the whole tile is one frozen chunk).
+// T tokens per tile. SOLVE: exact rule, else the tile is one frozen chunk.
 // States are stored at every tile start and after the last token.
 template <int RULE, bool SOLVE>
-__global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int rd)
+__global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
 {
     constexpr bool HAS_S = (RULE == RULE_TITANS);
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -329,17 +393,19 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
     float* Lb = reinterpret_cast<float*>(sm + F_E);      // Lx, fp32, until the solve is over
     const int tid = threadIdx.x, warp = uniform_warp();
     const int R = (warp & 3) * 32 + (tid & 31), hf = warp >> 2;     // TMEM lane, column half
+    const int dt = tid - 160;                                       // columns of the decay table: warps 5 to 7
     const int tr = R & 63;                                          // token (or state row) of this thread
     const bool krow = R < 64;                                       // K / M rows, else Q / S rows
     const int b = blockIdx.x;
-    const float* xg = (krow ? a.k : a.q) + (size_t)b * a.in_stride_tok * D + hf * 32;
-    const float* vg = a.v + (size_t)b * a.in_stride_tok * D + hf * 32;
+    const Unit un(warp, tid & 31);
+    const size_t su = (size_t)b * a.in_stride_tok * D + un.cc * 8;
     const float* alg = a.alpha + (size_t)b * a.in_stride_tok;
     const float* thg = a.theta + (size_t)b * a.in_stride_tok;
     const float* etg = HAS_S ? a.eta + (size_t)b * a.in_stride_tok : nullptr;
-    float* yg = a.y + (size_t)b * a.seq_len * D + hf * 32;
-    float* sg = (krow ? a.m_out : a.s_out);                         // this thread's state output
-    if (HAS_S || krow) sg += (size_t)b * a.out_stride + tr * D + hf * 32;
+    float* yg = a.y + (size_t)b * a.seq_len * D + un.cc * 8;
+    const size_t sgo = (size_t)b * a.out_stride + un.cc * 8;
+    float* Sb = reinterpret_cast<float*>(sm + F_EW);     // tile-end states on their way out, fp32
+    float* Yb = reinterpret_cast<float*>(sm + F_E);      // outputs on their way out, fp32
     const int ntile = (a.seq_len + T - 1) / T;
 
     if (tid == 0) { mbar_init(smem_u32(&tb.bar[0]), 1); mbar_init(smem_u32(&tb.bar[1]), 1); mbar_init(smem_u32(&tb.bar[2]), 1); }
@@ -357,14 +423,17 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
     if (HAS_S || krow) {
         ld32(st, (krow ? a.m_init : a.s_init) + (size_t)b * a.init_stride + tr * D + hf * 32, true);
         store32(sm + F_MS, 128, 16384, R, hf * 4, st);
-        st32(sg, st);
+        st32((krow ? a.m_out : a.s_out) + (size_t)b * a.out_stride + tr * D + hf * 32, st);
     }
-    float x[32], v[32], gal = 0.f, gth = 0.f, get = 0.f;
-    auto fetch = [&](int c) {         // this thread's rows and gates of tile c
+    float x[4][8], v[2][8], gal = 0.f, gth = 0.f, get = 0.f;
+    auto fetch = [&](int c) {         // this thread's units (K 0, 1, Q 2, 3, V) and gates of tile c
         const int t0 = c * T, L = min(T, a.seq_len - t0);
-        const bool ok = tr < L;
-        ld32(x, xg + (size_t)(t0 + tr) * D, ok);
-        if (krow) ld32(v, vg + (size_t)(t0 + tr) * D, ok);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = un.row(i & 1);
+            ld8_row(x[i], (i < 2 ? a.k : a.q) + su + (size_t)t0 * D, r, L);
+            if (i < 2) ld8_row(v[i], a.v + su + (size_t)t0 * D, r, L);
+        }
         if (tid < TMAX) {
             gal = (tid < L) ? alg[t0 + tid] : 0.f;
             gth = (tid < L) ? thg[t0 + tid] : 0.f;
@@ -375,7 +444,13 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
 
     for (int c = 0; c < ntile; c++) {
         const int t0 = c * T, L = min(T, a.seq_len - t0);
-        store32(sm + F_KQ, 128, 16384, R, hf * 4, x);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            zero_past(x[i], un.row(i & 1), L);
+            if (i < 2) zero_past(v[i], un.row(i), L);
+            store8(sm + F_KQ, 128, 16384, un.row(i), un.cc, x[i]);
+            if (i < 2) st8(Xb + un.row(i) * LDX + un.cc * 8, v[i]);
+        }
         if (tid < TMAX) tb.gt[tid] = make_float4(1.0f - gal, get, gth, 0.f);
         publish();
         if (warp == 0 && elect_one()) {
@@ -385,19 +460,11 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
             mma_commit(smem_u32(&tb.bar[0]));
         }
         float w[32], au, bu;
-        const int u = krow ? (tr / rd) * rd - 1 : tr;
-        decay_row(tb.gt, u, hf, w, au, bu);
-        if (R == 64 + L - 1) {
-#pragma unroll
-            for (int i = 0; i < 32; i++) tb.wM[hf * 32 + i] = w[i];
-            if (hf == 0) { tb.tot[0] = au; tb.tot[1] = bu; }
-        }
-        if (HAS_S && tid < TMAX) {
-            float hh = 1.f;
-            for (int i = L - 1; i > tid; i--) hh *= tb.gt[i].y;
-            tb.wS[tid] = (tid < L) ? tb.gt[tid].z * hh : 0.f;
-            if (tid == 0) tb.tot[2] = hh * tb.gt[0].y;
-        }
+        const int u = !krow ? tr : SOLVE ? tr - 1 : -1;
+        decay_table<HAS_S>(tb, Lb, dt, L);           // Lb is free until the scores are in
+        __syncthreads();
+        decay_row(tb, Lb, u, hf, w, au, bu);
+        __syncthreads();
         wait(0);
         float acc[32], p[32];
         tload(acc, trow);
@@ -411,7 +478,10 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
         tload(p, trow + 128);
         if (krow) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) acc[i] -= v[i];
+            for (int i = 0; i < 8; i++) {
+                const float4 v4 = *reinterpret_cast<const float4*>(Xb + tr * LDX + hf * 32 + 4 * i);
+                acc[4 * i] -= v4.x; acc[4 * i + 1] -= v4.y; acc[4 * i + 2] -= v4.z; acc[4 * i + 3] -= v4.w;
+            }
             st32(Xb + tr * LDX + hf * 32, acc);
             if (SOLVE) {
 #pragma unroll
@@ -426,27 +496,21 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
         if (c + 1 < ntile) fetch(c + 1);         // lands under the solve and the products
         __syncthreads();
         if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
-        {
-            // E and its tile-end weighted copies as planes
-            const int row = tid & 63, q = tid >> 6;
+        // E and its tile-end weighted copies as planes
+#pragma unroll 1
+        for (int i = 0; i < 2; i++) {
+            const int row = un.row(i);
             const float wm = tb.wM[row], wsv = HAS_S ? tb.wS[row] : 0.f;
-            float e[16], s[8];
+            float e[8], s[8];
+            ld8(e, Xb + row * LDX + un.cc * 8);
+            store8(sm + F_E, 64, 8192, row, un.cc, e);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
-                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
-            }
+            for (int j = 0; j < 8; j++) s[j] = e[j] * wm;
+            store8(sm + F_EW, 64, 16384, row, un.cc, s);
+            if (HAS_S) {
 #pragma unroll
-            for (int c8 = 0; c8 < 2; c8++) {
-                store8(sm + F_E, 64, 8192, row, 2 * q + c8, e + 8 * c8);
-#pragma unroll
-                for (int i = 0; i < 8; i++) s[i] = e[8 * c8 + i] * wm;
-                store8(sm + F_EW, 64, 16384, row, 2 * q + c8, s);
-                if (HAS_S) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) s[i] = e[8 * c8 + i] * wsv;
-                    store8(sm + F_EW, 64, 16384, row, 8 + 2 * q + c8, s);
-                }
+                for (int j = 0; j < 8; j++) s[j] = e[j] * wsv;
+                store8(sm + F_EW, 64, 16384, row, 8 + un.cc, s);
             }
         }
         publish();
@@ -478,14 +542,22 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T, int r
 #pragma unroll
             for (int i = 0; i < 32; i++) st[i] -= p[i];
             store32(sm + F_MS, 128, 16384, R, hf * 4, st);
-            st32(sg + (size_t)(c + 1) * DD, st);
+            st32(Sb + R * LDX + hf * 32, st);          // the weighted errors have been consumed
         }
         wait(2);
         tload(p, trow + 192);
-        if (!krow && tr < L) {
+        if (!krow) {
 #pragma unroll
             for (int i = 0; i < 32; i++) p[i] += acc[i];
-            st32(yg + (size_t)(t0 + tr) * D, p);
+            st32(Yb + tr * LDX + hf * 32, p);          // and so have the errors
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int r = un.row(i);
+            copy8(a.m_out + sgo + (size_t)(c + 1) * DD + r * D, Sb + r * LDX + un.cc * 8);
+            if (HAS_S) copy8(a.s_out + sgo + (size_t)(c + 1) * DD + r * D, Sb + (64 + r) * LDX + un.cc * 8);
+            if (r < L) copy8(yg + (size_t)(t0 + r) * D, Yb + r * LDX + un.cc * 8);
         }
     }
     if (wait.dead && (tid & 31) == 0) atomicExch(&g_mtc_timeout, 1);
@@ -503,31 +575,32 @@ constexpr int BWD_SMEM = B_TAB + (int)sizeof(Tables);
 // trajectory, no S stored): S at a tile start is M_t - (1 - alpha_{t-1}) M_{t-1}, and at the first token
 // (M_1 - r_0 M_0 + theta_0 e_0 k_0^T) / eta_0.
 template <int RULE, bool SOLVE, bool SDER>
-__global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int rd, long long mstep)
+__global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long long mstep)
 {
     constexpr bool HAS_S = (RULE == RULE_TITANS);
     extern __shared__ __align__(1024) unsigned char sm[];
     Tables& tb = *reinterpret_cast<Tables*>(sm + B_TAB);
     float* Xb = reinterpret_cast<float*>(sm + B_WZ);                  // right-hand sides, fp32
     float* Lb = reinterpret_cast<float*>(sm + B_WZ + TMAX * LDX * 4);     // Lx, fp32
+    float* Ob = Xb + 2 * TMAX * LDX;                                  // dK and dQ on their way out, fp32
     float* Sd = reinterpret_cast<float*>(sm + B_X);                   // scan buffers X -> Xd, and Xs
     float* Ss = reinterpret_cast<float*>(sm + B_X + 17408);
     float* Gx = reinterpret_cast<float*>(sm + B_E);                   // G_M rows for the S rows
     const int tid = threadIdx.x, warp = uniform_warp(), lane = tid & 31;
     const int R = (warp & 3) * 32 + lane, hf = warp >> 2;
+    const int dt = tid - 160;          // columns of the decay table: warps 5 to 7
     const int tr = R & 63;
     const bool krow = R < 64;
     const int b = blockIdx.x;
-    const size_t so = (size_t)b * a.seq_len * D + hf * 32, go = (size_t)b * a.seq_len;
-    const float* xg = (krow ? a.k : a.q) + so;
-    const float* yg = (krow ? a.v : a.d_y) + so;
+    const Unit un(warp, lane);
+    const size_t so = (size_t)b * a.seq_len * D, go = (size_t)b * a.seq_len;
+    const size_t su = so + un.cc * 8;
     const float* mtraj = a.m_traj + (size_t)b * a.traj_stride;
     const float* straj = (HAS_S && !SDER) ? a.s_traj + (size_t)b * a.traj_stride : nullptr;
-    float* dxg = (krow ? a.d_k : a.d_q) + so;
     const int n = a.t_end - a.t_start;
     const int ntile = (n + T - 1) / T;
 
-    if (tid == 0) mbar_init(smem_u32(&tb.bar[0]), 1);
+    if (tid == 0) { mbar_init(smem_u32(&tb.bar[0]), 1); mbar_init(smem_u32(&tb.bar[1]), 1); }
     if (warp == 0) tmem_alloc_cols(reinterpret_cast<unsigned char*>(&tb.tmem), TCOLS);
     fence_before_sync();
     __syncthreads();
@@ -550,51 +623,63 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
     for (int c = ntile - 1; c >= 0; c--) {
         const int t0 = a.t_start + c * T, L = min(T, n - c * T);
         const bool ok = tr < L;
-        auto state_row = [&](float (&x3)[32]) {      // this thread's row of M0 or S0
+        auto state_unit = [&](float (&x3)[8], int i) {   // unit i of M0 (0, 1) or S0 (2, 3)
             const float* mp = mtraj + (size_t)c * mstep;
-            if (krow) ld32(x3, mp + tr * D + hf * 32, true);
-            else if (HAS_S && !SDER) ld32(x3, straj + (size_t)c * mstep + tr * D + hf * 32, true);
+            const int r = un.row(i & 1), ofs = r * D + un.cc * 8;
+            if (i < 2) ld8(x3, mp + ofs);
+            else if (HAS_S && !SDER) ld8(x3, straj + (size_t)c * mstep + ofs);
             else if (SDER) {
                 const float* m1 = (c > 0) ? mp : mp + DD;
                 const float* m0 = (c > 0) ? mp - DD : mp;
                 const int ta = (c > 0) ? t0 - 1 : t0;
-                const float r = 1.0f - a.alpha[go + ta];
-                float y3[32];
-                ld32(x3, m1 + tr * D + hf * 32, true);
-                ld32(y3, m0 + tr * D + hf * 32, true);
+                const float rr = 1.0f - a.alpha[go + ta];
+                float y3[8];
+                ld8(x3, m1 + ofs);
+                ld8(y3, m0 + ofs);
 #pragma unroll
-                for (int i = 0; i < 32; i++) x3[i] = fmaf(-r, y3[i], x3[i]);
+                for (int j = 0; j < 8; j++) x3[j] = fmaf(-rr, y3[j], x3[j]);
                 if (c == 0) {
-                    const float* k0 = a.k + (so - hf * 32) + (size_t)t0 * D;
-                    float e = -a.v[(so - hf * 32) + (size_t)t0 * D + tr];
-                    for (int j = 0; j < D; j++) e = fmaf(m0[tr * D + j], k0[j], e);
+                    const float* k0 = a.k + so + (size_t)t0 * D;
+                    float e = -a.v[so + (size_t)t0 * D + r];
+#pragma unroll 4
+                    for (int j = 0; j < D; j++) e = fmaf(m0[r * D + j], k0[j], e);
                     const float te = a.theta[go + t0] * e, et = a.eta[go + t0];
                     const float inv = et > 1e-30f ? 1.0f / et : 0.f;
 #pragma unroll
-                    for (int i = 0; i < 32; i++) x3[i] = fmaf(te, k0[hf * 32 + i], x3[i]) * inv;
+                    for (int j = 0; j < 8; j++) x3[j] = fmaf(te, k0[un.cc * 8 + j], x3[j]) * inv;
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < 32; i++) x3[i] = 0.f;
+                for (int j = 0; j < 8; j++) x3[j] = 0.f;
             }
         };
         // ── stage 1: operands; K K^T | Q K^T and K,Q x M0,S0 ──
-        float y[32];                                 // V row (krow) or dY row
+        // The four units of each matrix go round one loop, the next unit's loads in flight: straight-line
+        // code is fetched once per tile by every warp and was bound by that (8k cycles against 4k).
         {
-            float x[32];
-            ld32(x, xg + (size_t)(t0 + tr) * D, ok);
-            ld32(y, yg + (size_t)(t0 + tr) * D, ok);
-            store32(kqp, 128, 16384, R, hf * 4, x);
-            if (!krow) store32(yfp, 128, 16384, R, hf * 4, y);
-        }
-        float dots[2];
-        {
-            float x3[32];
-            state_row(x3);
-            store32(xxp, 128, 16384, R, hf * 4, x3);
-            dots[0] = 0.f;
+            float x[8], y[8], x3[8];
+            auto get = [&](int i) {                  // K, V, M0 rows, then Q, dY, S0 rows
+                const int r = un.row(i & 1);
+                ld8_row(x, (i < 2 ? a.k : a.q) + su + (size_t)t0 * D, r, L);
+                ld8_row(y, (i < 2 ? a.v : a.d_y) + su + (size_t)t0 * D, r, L);
+                state_unit(x3, i);
+            };
+            get(0);
+#pragma unroll 1
+            for (int i = 0; i < 4; i++) {
+                float xc[8], yc[8], x3c[8];
+                const int r = un.row(i);
 #pragma unroll
-            for (int i = 0; i < 32; i++) dots[0] = fmaf(g[i], x3[i], dots[0]);     // <M0,G_M> or <S0,G_S>
+                for (int j = 0; j < 8; j++) {
+                    const bool in = un.row(i & 1) < L;
+                    xc[j] = in ? x[j] : 0.f; yc[j] = in ? y[j] : 0.f; x3c[j] = x3[j];
+                }
+                if (i < 3) get(i + 1);
+                store8(kqp, 128, 16384, r, un.cc, xc);
+                store8(xxp, 128, 16384, r, un.cc, x3c);
+                if (i < 2) st8(Xb + r * LDX + un.cc * 8, yc);
+                else store8(yfp, 128, 16384, r, un.cc, yc);
+            }
         }
         if (tid < TMAX) {
             const bool in = tid < L;
@@ -608,32 +693,36 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
             mma6<false, false>(tm + 64, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);
             mma_commit(smem_u32(&tb.bar[0]));
         }
+        if (c > 0 && tid < 4) {                       // the next tile's streams, while this one is worked on
+            const float* nx = (tid == 0 ? a.k : tid == 1 ? a.q : tid == 2 ? a.v : a.d_y) + so + (size_t)(t0 - T) * D;
+            l2_prefetch(nx, (unsigned)T * D * 4);
+        } else if (c > 0 && tid < 6) {
+            if (tid == 4) l2_prefetch(mtraj + (size_t)(c - 1) * mstep, DD * 4);
+            else if (straj != nullptr) l2_prefetch(straj + (size_t)(c - 1) * mstep, DD * 4);
+            else if (SDER && c > 1) l2_prefetch(mtraj + (size_t)(c - 1) * mstep - DD, DD * 4);
+        }
         float w[32], p[32], au, bu;
-        const int u = krow ? (tr / rd) * rd - 1 : tr;
-        decay_row(tb.gt, u, hf, w, au, bu);
-        if (R == 64 + L - 1) {
+        const int u = !krow ? tr : SOLVE ? tr - 1 : -1;
+        float dots[2] = {0.f, 0.f};                   // <M0, G_M> or <S0, G_S>; <S0, G_M>
 #pragma unroll
-            for (int i = 0; i < 32; i++) tb.wM[hf * 32 + i] = w[i];
-            if (hf == 0) { tb.tot[0] = au; tb.tot[1] = bu; }
-        }
-        if (HAS_S && tid < TMAX) {
-            float hh = 1.f;
-            for (int i = L - 1; i > tid; i--) hh *= tb.gt[i].y;
-            tb.wS[tid] = (tid < L) ? tb.gt[tid].z * hh : 0.f;
-            if (tid == 0) tb.tot[2] = hh * tb.gt[0].y;
-        }
-        dots[1] = 0.f;
-        if (HAS_S && krow) {                          // <S0, G_M>
+        for (int c8 = 0; c8 < 4; c8++) {
+            float m[8];
+            if (HAS_S || krow) {
+                load8(m, xxp, 128, 16384, R, hf * 4 + c8);
 #pragma unroll
-            for (int c8 = 0; c8 < 4; c8++) {
-                float s[8];
-                load8(s, xxp, 128, 16384, 64 + tr, hf * 4 + c8);
+                for (int i = 0; i < 8; i++) dots[0] = fmaf(g[8 * c8 + i], m[i], dots[0]);
+            }
+            if (HAS_S && krow) {
+                load8(m, xxp, 128, 16384, 64 + tr, hf * 4 + c8);
 #pragma unroll
-                for (int i = 0; i < 8; i++) dots[1] = fmaf(g[8 * c8 + i], s[i], dots[1]);
+                for (int i = 0; i < 8; i++) dots[1] = fmaf(g[8 * c8 + i], m[i], dots[1]);
             }
         }
+        decay_table<HAS_S>(tb, Gx, dt, L);            // the errors' planes are free until stage 2
         dots[0] = warp_sum(dots[0]); dots[1] = warp_sum(dots[1]);
         if (lane == 0) { tb.red[warp][0] = dots[0]; tb.red[warp][1] = dots[1]; }
+        __syncthreads();
+        decay_row(tb, Gx, u, hf, w, au, bu);
         wait(0);
         tload(p, trow);                               // k_t . k_j or q_t . k_j
         {
@@ -641,7 +730,11 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
             tload(acc, trow + 64);
             if (krow) {
 #pragma unroll
-                for (int i = 0; i < 32; i++) acc[i] = fmaf(au, acc[i], -y[i]);
+                for (int i = 0; i < 8; i++) {
+                    const float4 v4 = *reinterpret_cast<const float4*>(Xb + tr * LDX + hf * 32 + 4 * i);
+                    acc[4 * i] = fmaf(au, acc[4 * i], -v4.x); acc[4 * i + 1] = fmaf(au, acc[4 * i + 1], -v4.y);
+                    acc[4 * i + 2] = fmaf(au, acc[4 * i + 2], -v4.z); acc[4 * i + 3] = fmaf(au, acc[4 * i + 3], -v4.w);
+                }
                 if (HAS_S) {
                     float s[32];
                     tload(s, trow + 128);
@@ -655,7 +748,9 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                     st32(Lb + tr * LDX + hf * 32, acc);
                 }
             } else {
-                float zm = 0.f, zs = 0.f;
+                float zm = 0.f, zs = 0.f, y[32];
+#pragma unroll
+                for (int c8 = 0; c8 < 4; c8++) load8(y + 8 * c8, yfp, 128, 16384, R, hf * 4 + c8);
 #pragma unroll
                 for (int i = 0; i < 32; i++) zm = fmaf(y[i], acc[i], zm);
                 if (HAS_S) {
@@ -669,16 +764,11 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
         __syncthreads();
         if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
         // ── stage 2: E planes, W o P, G planes; right-hand side of F, E x G ──
-        {
-            const int row = tid & 63, q = tid >> 6;
-            float e[16];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
-                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
-            }
-            store8(sm + B_E, 64, 8192, row, 2 * q, e);
-            store8(sm + B_E, 64, 8192, row, 2 * q + 1, e + 8);
+#pragma unroll 1
+        for (int i = 0; i < 2; i++) {
+            float e[8];
+            ld8(e, Xb + un.row(i) * LDX + un.cc * 8);
+            store8(sm + B_E, 64, 8192, un.row(i), un.cc, e);
         }
         if (!krow) {
             float wpv[32];
@@ -692,12 +782,11 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
             fence_after_sync();
             mma6<false, false>(tm, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);              // K G^T
             mma6<true, true>(tm + 128, wz + 24576, 8192, 64, yf + 1024, 16384, 128, 64, 4);           // (W o P)^T dY
+            mma_commit(smem_u32(&tb.bar[0]));
             mma6<false, true>(tm + 192, ep, 8192, 64, xx, 16384, 128, 64, 4);                         // E G_M
             if (HAS_S) mma6<false, true>(tm + 256, ep, 8192, 64, xx + 1024, 16384, 128, 64, 4);       // E G_S
-            mma_commit(smem_u32(&tb.bar[0]));
+            mma_commit(smem_u32(&tb.bar[1]));
         }
-        float x3[32];
-        state_row(x3);
         wait(0);
         float dx[32];                                  // gradient of this thread's K or Q row
         if (krow) {
@@ -718,68 +807,74 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                 for (int i = 0; i < 32; i++) s[i] = w[i] * p[i];
                 st32(Lb + tr * LDX + hf * 32, s);
             }
-            float gm = 0.f, gs = 0.f;
+        }
+        __syncthreads();
+        if (SOLVE) solve_lower_t(Lb, Xb, (L + 15) >> 4);
+        wait(1);
+        if (krow) {
+            const float wm = tb.wM[tr], wsv = HAS_S ? tb.wS[tr] : 0.f;
+            float gm = 0.f, gs = 0.f, s[32], s2[32];
             tload(s, trow + 192);
-#pragma unroll
-            for (int i = 0; i < 32; i++) dx[i] = -wm * s[i];
+            if (HAS_S) tload(s2, trow + 256);
 #pragma unroll
             for (int c8 = 0; c8 < 4; c8++) {
                 float kk[8];
                 load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
 #pragma unroll
-                for (int i = 0; i < 8; i++) gm = fmaf(kk[i], s[8 * c8 + i], gm);
-            }
-            if (HAS_S) {
-                tload(s, trow + 256);
-#pragma unroll
-                for (int i = 0; i < 32; i++) dx[i] = fmaf(-wsv, s[i], dx[i]);
-#pragma unroll
-                for (int c8 = 0; c8 < 4; c8++) {
-                    float kk[8];
-                    load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) gs = fmaf(kk[i], s[8 * c8 + i], gs);
+                for (int i = 0; i < 8; i++) {
+                    gm = fmaf(kk[i], s[8 * c8 + i], gm);
+                    if (HAS_S) gs = fmaf(kk[i], s2[8 * c8 + i], gs);
                 }
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i++) {
+                dx[i] = -wm * s[i];
+                if (HAS_S) dx[i] = fmaf(-wsv, s2[i], dx[i]);
             }
             tb.z[2][hf * 64 + tr] = gm; tb.z[3][hf * 64 + tr] = gs;
         }
-        __syncthreads();
-        if (SOLVE) solve_lower_t(Lb, Xb, (L + 15) >> 4);
         // ── stage 3: F planes, dV, M0/S0 planes again; N | R, F and dY x M0,S0 ──
-        {
-            const int row = tid & 63, q = tid >> 6;
-            float e[16];
+#pragma unroll 1
+        for (int i = 0; i < 2; i++) {
+            const int r = un.row(i);
+            float e[8];
+            ld8(e, Xb + r * LDX + un.cc * 8);
+            store8(yfp, 128, 16384, r, un.cc, e);
+            if (r < L) {
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 t4 = *reinterpret_cast<const float4*>(Xb + row * LDX + 16 * q + 4 * i);
-                e[4 * i] = t4.x; e[4 * i + 1] = t4.y; e[4 * i + 2] = t4.z; e[4 * i + 3] = t4.w;
-            }
-            store8(yfp, 128, 16384, row, 2 * q, e);
-            store8(yfp, 128, 16384, row, 2 * q + 1, e + 8);
-            if (row < L) {
-                float* dv = a.d_v + (so - hf * 32) + (size_t)(t0 + row) * D + 16 * q;
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    *reinterpret_cast<float4*>(dv + 4 * i) = make_float4(-e[4 * i], -e[4 * i + 1], -e[4 * i + 2], -e[4 * i + 3]);
+                for (int j = 0; j < 8; j++) e[j] = -e[j];
+                st8(a.d_v + su + (size_t)(t0 + r) * D, e);
             }
         }
-        store32(xxp, 128, 16384, R, hf * 4, x3);
+        {
+            float x3[8];
+            state_unit(x3, 0);
+#pragma unroll 1
+            for (int i = 0; i < 4; i++) {
+                float x3c[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) x3c[j] = x3[j];
+                if (i < 3) state_unit(x3, i + 1);
+                store8(xxp, 128, 16384, un.row(i), un.cc, x3c);
+            }
+        }
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, yf, 16384, 128, ep, 8192, 64, 64, 4);                       // F,dY x E
+            mma_commit(smem_u32(&tb.bar[0]));
             mma6<false, true>(tm + 64, yf, 16384, 128, xx, 16384, 128, 64, 4);                 // F,dY x M0
             if (HAS_S) mma6<false, true>(tm + 128, yf, 16384, 128, xx + 1024, 16384, 128, 64, 4);   // F,dY x S0
-            mma_commit(smem_u32(&tb.bar[0]));
+            mma_commit(smem_u32(&tb.bar[1]));
         }
         wait(0);
-        float zkm = 0.f, zks = 0.f;
         {
             float s[32];
             tload(s, trow);                            // N row (krow) or R row
 #pragma unroll
             for (int i = 0; i < 32; i++) { p[i] *= s[i]; s[i] *= -w[i]; }
             store32(sm + B_WZ, 128, 16384, R, hf * 4, s);
+            wait(1);
             if (!krow) {
                 // every read of the state planes by the tensor cores is over: the scan buffers take their place
 #pragma unroll
@@ -787,41 +882,32 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                 if (hf == 0) Sd[tr * LDS + 64] = tb.z[0][tr] + tb.z[0][64 + tr];
                 else Sd[tr * LDS + 65] = tb.z[1][tr] + tb.z[1][64 + tr];
             }
+            float s2[32];
             tload(s, trow + 64);
-            if (krow) {
+            if (HAS_S) tload(s2, trow + 128);
+            if (SOLVE && krow) {
+                float zkm = 0.f, zks = 0.f;
 #pragma unroll
-                for (int i = 0; i < 32; i++) dx[i] = fmaf(au, s[i], dx[i]);
-                if (SOLVE) {
+                for (int c8 = 0; c8 < 4; c8++) {
+                    float kk[8];
+                    load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
 #pragma unroll
-                    for (int c8 = 0; c8 < 4; c8++) {
-                        float kk[8];
-                        load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
-#pragma unroll
-                        for (int i = 0; i < 8; i++) zkm = fmaf(kk[i], s[8 * c8 + i], zkm);
+                    for (int i = 0; i < 8; i++) {
+                        zkm = fmaf(kk[i], s[8 * c8 + i], zkm);
+                        if (HAS_S) zks = fmaf(kk[i], s2[8 * c8 + i], zks);
                     }
                 }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; i++) dx[i] = au * s[i];
+                tb.part[0][hf * 64 + tr] = zkm; tb.part[1][hf * 64 + tr] = zks;
             }
-            if (HAS_S) {
-                tload(s, trow + 128);
 #pragma unroll
-                for (int i = 0; i < 32; i++) dx[i] = fmaf(bu, s[i], dx[i]);
-                if (SOLVE && krow) {
-#pragma unroll
-                    for (int c8 = 0; c8 < 4; c8++) {
-                        float kk[8];
-                        load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
-#pragma unroll
-                        for (int i = 0; i < 8; i++) zks = fmaf(kk[i], s[8 * c8 + i], zks);
-                    }
-                }
+            for (int i = 0; i < 32; i++) {
+                dx[i] = krow ? fmaf(au, s[i], dx[i]) : au * s[i];
+                if (HAS_S) dx[i] = fmaf(bu, s2[i], dx[i]);
             }
         }
         publish();
         // ── stage 4: (W o R, Z) x K and transposes; gate scans under them ──
-        if (warp == 0 && elect_one()) {
+        if (warp == 4 && elect_one()) {                // warps 0 to 2 have the scans to do
             fence_after_sync();
             mma6<false, true>(tm + 192, wz, 16384, 128, kq, 16384, 128, 64, 4);        // rows: Z K | -(W o R) K
             mma6<true, true>(tm + 256, wz, 16384, 128, kq, 16384, 128, 64, 8);         // Z^T K - (W o R)^T Q
@@ -829,15 +915,10 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
         }
         if (SOLVE) {
             if (krow && u >= 0 && ok) {
-                if (rd == 1) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) Sd[u * LDS + hf * 32 + i] += p[i];
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i++) atomicAdd(&Sd[u * LDS + hf * 32 + i], p[i]);
-                }
-                atomicAdd(&Sd[u * LDS + 64], zkm);
-                if (HAS_S) atomicAdd(&Sd[u * LDS + 65], zks);
+                for (int i = 0; i < 32; i++) Sd[u * LDS + hf * 32 + i] += p[i];
+                // the M0 and S0 columns take the error's share too
+                Sd[u * LDS + 64 + hf] += tb.part[hf][tr] + tb.part[hf][64 + tr];
             }
             __syncthreads();
         }
@@ -855,13 +936,25 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                     if (j == 65 && !kw) sS += tb.red[wq][0];
                 }
             }
-            float xd = sM, xs = sS;
-            for (int s = L - 1; s >= 0; s--) {
-                const float4 gn = (s + 1 < L) ? tb.gt[s + 1] : make_float4(1.f, 1.f, 0.f, 0.f);
-                xd = fmaf(gn.x, xd, Sd[s * LDS + j]);
-                xs = fmaf(gn.y, xs, xd);
-                Sd[s * LDS + j] = xd;
-                Ss[s * LDS + j] = xs;
+            float xd = sM, xs = sS, gr = 1.f, ge = 1.f;      // r and eta of the row above
+#pragma unroll 1
+            for (int s0 = 48; s0 >= 0; s0 -= 16) {
+                if (s0 >= L) continue;
+                float xv[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) xv[i] = Sd[(s0 + i) * LDS + j];
+#pragma unroll
+                for (int i = 15; i >= 0; i--) {
+                    const float4 gn = tb.gt[s0 + i];
+                    const bool in = s0 + i < L;            // rows past the tile are written but never read
+                    xd = in ? fmaf(gr, xd, xv[i]) : xd;
+                    xs = in ? fmaf(ge, xs, xd) : xs;
+                    gr = in ? gn.x : 1.f; ge = in ? gn.y : 1.f;
+                    xv[i] = xd;
+                    Ss[(s0 + i) * LDS + j] = xs;
+                }
+#pragma unroll
+                for (int i = 0; i < 16; i++) Sd[(s0 + i) * LDS + j] = xv[i];
             }
             if (j < L) a.d_theta[go + t0 + j] = -Ss[j * LDS + j];
         }
@@ -876,9 +969,18 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                 for (int i = 0; i < 32; i++) s1 = fmaf(w[i], xd[i], s1);     // w is zero above the diagonal
                 if (HAS_S) {
                     float hh = 1.f;
-                    for (int j = tr; j >= 0; j--) {
-                        if (j < tr) hh *= tb.gt[j + 1].y;
-                        if ((j >> 5) == hf) s2 = fmaf(tb.gt[j].z * hh, xs[j - hf * 32], s2);
+                    const int jh = hf * 32;
+                    float4 gn = tb.gt[hf == 0 ? 32 : 63];          // gates of column j + 1
+                    if (hf == 0) {
+#pragma unroll 8
+                        for (int j = 62; j >= 32; j--) { const float et = tb.gt[j + 1].y; hh = (j < tr) ? hh * et : hh; }
+                    }
+#pragma unroll 8
+                    for (int j = 31; j >= 0; j--) {
+                        const float4 gj = tb.gt[jh + j];
+                        hh = (jh + j < tr) ? hh * gn.y : hh;
+                        s2 = (jh + j <= tr) ? fmaf(gj.z * hh, xs[j], s2) : s2;
+                        gn = gj;
                     }
                     hend = hh * tb.gt[0].y;
                 }
@@ -908,11 +1010,10 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
 #pragma unroll
                 for (int i = 0; i < 32; i++) dx[i] += s[i];
             }
-            if (ok) st32(dxg + (size_t)(t0 + tr) * D, dx);
         }
         __syncthreads();                               // the scan buffers have been read
         // ── stage 5: carry. [diag(a) F ; diag(A) dY | diag(b) F ; diag(B) dY]^T [K ; Q] ──
-#pragma unroll
+#pragma unroll 1
         for (int c8 = 0; c8 < 4; c8++) {
             float f[8], s[8];
             load8(f, yfp, 128, 16384, R, hf * 4 + c8);
@@ -949,8 +1050,15 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, int r
                 for (int i = 0; i < 32; i++) g[i] += s[i];
             }
         }
+        st32(Ob + R * LDX + hf * 32, dx);
         fence_before_sync();
         __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = un.row(i & 1);
+            if (r < L) copy8((i < 2 ? a.d_k : a.d_q) + su + (size_t)(t0 + r) * D, Ob + un.row(i) * LDX + un.cc * 8);
+        }
+        __syncthreads();                               // the next tile's planes go over the staged rows
     }
 
     if ((HAS_S || krow) && a.d_m_out != nullptr) {
