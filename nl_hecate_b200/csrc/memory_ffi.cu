@@ -92,16 +92,6 @@ static int run_forward(int rule, FwdArgs a, const char* where)
     return ok ? NLH_OK : NLH_ERR_CUDA;
 }
 
-// Backward in matrix form on the tensor cores. Stored states: chunk / checkpoint boundaries (a.chunk
-// tokens apart) or every state, of which only one per tile is read. A tile costs about as much as 24
-// tokens of the per-token kernels, whatever its length: shorter ranges stay with those.
-static bool tile_backward(int rule, const BwdArgs& a, cudaStream_t st)
-{
-    const long long dd = (long long)a.d * a.d;
-    if (a.chunk > 0) return mtc::backward(rule, a, a.chunk, dd, st);
-    return !a.frozen && a.t_end - a.t_start >= 24 && mtc::backward(rule, a, 64, 64 * dd, st);
-}
-
 static int run_backward(int rule, BwdArgs a, const char* where)
 {
     if (!valid_dims(where, a.seq_len, a.d, a.batch)) return NLH_ERR_INVALID_ARG;
@@ -111,7 +101,7 @@ static int run_backward(int rule, BwdArgs a, const char* where)
         return NLH_ERR_INVALID_ARG;
     }
     cudaStream_t st = current_stream();
-    if (option_value(NLH_OPT_CHUNK_MATRIX) && tile_backward(rule, a, st))
+    if (option_value(NLH_OPT_CHUNK_MATRIX) && mtc::backward(rule, a, st))
         return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (fast_backward(rule, a, st)) return check_launch(where) ? NLH_OK : NLH_ERR_CUDA;
     if (rule == RULE_TITANS && a.s_traj == nullptr) {

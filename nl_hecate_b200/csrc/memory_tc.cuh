@@ -1,39 +1,39 @@
-// Titans / Delta memory rule in CHUNK-PARALLEL (matrix) form on the 5th-generation tensor cores,
-// head dimension 64: exact rule, and frozen-M0 rule with one chunk per tile.
+// Frozen-M0 chunkwise Titans / Delta rule in CHUNK-PARALLEL (matrix) form on the 5th-generation tensor
+// cores, head dimension 64.
 //
-// A problem's tokens are cut into tiles of up to 64. Inside a tile everything is linear in the
-// tile-start state (M0, S0) and the errors E (rows e_t). With r_t = 1 - alpha_t and, for t >= j,
+// A problem's tokens are cut into tiles of one chunk, up to 64. Inside a tile the errors come from the
+// tile-start state (M0, S0) and everything is linear in it and in them (E: rows e_t). With r_t = 1 - alpha_t
+// and, for t >= j,
 //     h(j,t)  = prod_{i=j+1..t} eta_i ,  rho(j,t) = prod_{i=j+1..t} r_i
 //     Om(t,j) = sum_{i=j..t} h(j,i) rho(i,t)        (weight of -theta_j e_j k_j^T in the state M_t)
 //     A_t = prod_{i<=t} r_i,  H_t = prod_{i<=t} eta_i,  B_t = eta_0 Om(t,0)   (weights of M0, S0)
 //     W(t,j) = theta_j Om(t,j)
-// the state after token t is  M_t = A_t M0 + B_t S0 - sum_{j<=t} W(t,j) e_j k_j^T. The error of
-// token t is read from the state of index u(t): t-1 for the exact rule, -1 (the tile-start state) for
-// the frozen rule. With a_t = A_u, b_t = B_u (1, 0 for u = -1)
-//     (I + Lx) E = diag(a) K M0^T + diag(b) K S0^T - V ,   Lx(t,j) = W(u(t),j) (k_t . k_j)
-//     Y   = diag(A) Q M0^T + diag(B) Q S0^T - (W o P) E ,  P = Q K^T
+//     E   = K M0^T - V ,  P = Q K^T
+//     Y   = diag(A) Q M0^T + diag(B) Q S0^T - (W o P) E
 //     M_C = A_L M0 + B_L S0 - E^T diag(W(L-1,:)) K ,       S_C = H_L S0 - E^T diag(theta_j h(j,L-1)) K
 // and backward (G_M, G_S: gradients of the tile-end states)
-//     (I + Lx)^T F = -[ (W o P)^T dY + diag(W(L-1,:)) K G_M^T + diag(theta h) K G_S^T ] ,  dV = -F
-//     R = dY E^T ,  N = F E^T ,  Z = -W(u,:) o N
+//     F = -[ (W o P)^T dY + diag(W(L-1,:)) K G_M^T + diag(theta h) K G_S^T ] ,  dV = -F ,  R = dY E^T
 //     dQ  = diag(A) dY M0 + diag(B) dY S0 - (W o R) K
-//     dK  = diag(a) F M0 + diag(b) F S0 - diag(W(L-1,:)) E G_M - diag(theta h) E G_S + (Z + Z^T) K - (W o R)^T Q
-//     G_M' = dY^T diag(A) Q + F^T diag(a) K + A_L G_M
-//     G_S' = dY^T diag(B) Q + F^T diag(b) K + B_L G_M + H_L G_S
+//     dK  = F M0 - diag(W(L-1,:)) E G_M - diag(theta h) E G_S - (W o R)^T Q
+//     G_M' = dY^T diag(A) Q + F^T K + A_L G_M ,            G_S' = dY^T diag(B) Q + B_L G_M + H_L G_S
 // The gate gradients contract the states with their adjoints and reduce to two decayed scans down
-// the columns of X(s,j) = R(s,j) P(s,j) + sum_{t: u(t)=s} N(t,j) (k_t . k_j), plus two columns for M0
-// and S0. Only W's recurrences over tokens are sequential, and they are 64 scalar steps.
-// Same semantics as the per-token statements core/kernels/titans_forward.cu:83-199,
-// titans_backward.cu:66-345 and titans_chunkwise_{forward,backward}.cu.
+// the columns of X = R o P, plus two columns for M0 and S0. Only W's recurrences over tokens are
+// sequential, and they are 64 scalar steps.
+// Same semantics as the per-token statement core/kernels/titans_chunkwise_{forward,backward}.cu.
 //
 // Precision. Operands are fp32 and stay so: each is stored as THREE bf16 planes x = hi + mid + lo,
 // which hold all 24 bits of the significand, and a product is the six plane products
 // hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi accumulated in fp32 in TMEM, the small ones first (the
-// dropped ones are below 2^-24 of the product). Triangular solves, scans and gate tables are fp32 FMA.
+// dropped ones are below 2^-24 of the product). Scans and gate tables are fp32 FMA. Against float64, 16
+// problems x 333 tokens, chunk 64: y 1.25e-7, dK 2.0e-7, dV 1.8e-7, d_eta 2.0e-7 (fp32 FMA contractions, which
+// these replace: 1.6e-7, 3.1e-7, 2.1e-7, 2.4e-7). The exact rule has the same form with a triangular solve per
+// tile, but there it replaces per-token kernels at 1.0e-7 and came to 2.1e-7: it stays with those.
 //
 // What bounds it. One CTA (256 threads) walks one problem, so a launch is bound by the chain of a
-// tile's stages: tensor products (48 cycles per 128x64x16 plane product at the shared-memory read
-// rate), the conversion of every intermediate into planes, and the 64-row triangular solves.
+// tile's stages: tensor products (55 cycles per 128x64x16 plane product, the A operand is read from
+// shared memory for each; 22k of a backward tile's cycles), loads and the conversion of every intermediate
+// into planes with two warps per scheduler. The stage times are the same with 4 problems as with 128, so
+// neither memory nor the other SMs bound them.
 //
 // Shared-memory matrices: element (row, col) of an R-row plane at (col/8)*(R*16) + row*16 + (col%8)*2,
 // the canonical no-swizzle core-matrix layout with the 8-column chunk outermost. The same bytes serve
@@ -53,7 +53,7 @@ using namespace nlh::tc;
 constexpr int D = 64, DD = D * D;
 constexpr int TMAX = 64;          // tokens per tile
 constexpr int NT = 256;
-constexpr int LDX = 68;           // leading dimension of the fp32 solve buffers
+constexpr int LDX = 68;           // leading dimension of the fp32 staging buffers
 constexpr int LDS = 67;           // leading dimension of the scan buffers (64 columns + M0 + S0)
 constexpr unsigned TCOLS = 512;
 constexpr int MIN_TILE = 16;      // shorter tiles run the per-token register kernels
@@ -106,11 +106,11 @@ __device__ __forceinline__ void store32(unsigned char* t, int R, int plane, int 
 }
 
 // ── tensor product of split operands, issued by one thread ──
-// D[128, N] (+)= A B with contraction length 16 * ksteps. a_mn / b_mn: the operand's rows are the
+// D[128, N] (+)= A B with contraction length 16 * KSTEPS. a_mn / b_mn: the operand's rows are the
 // contraction index (MN-major), otherwise its rows are the M / N index (K-major).
-template <bool AMN, bool BMN>
+template <bool AMN, bool BMN, int KSTEPS = 4>
 __device__ __forceinline__ void mma6(unsigned d, unsigned a, int a_plane, int a_R, unsigned b, int b_plane, int b_R,
-                                     int N, int ksteps)
+                                     int N)
 {
     const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((AMN ? 1u : 0u) << 15) | ((BMN ? 1u : 0u) << 16) |
                            ((unsigned)(N >> 3) << 17) | (8u << 24);
@@ -125,7 +125,7 @@ __device__ __forceinline__ void mma6(unsigned d, unsigned a, int a_plane, int a_
         const unsigned pb = p == 1 ? 2u : (p == 2 || p == 4) ? 1u : 0u;
         const unsigned a0 = a + pa * a_plane, b0 = b + pb * b_plane;
 #pragma unroll 4
-        for (int k = 0; k < ksteps; k++) {
+        for (int k = 0; k < KSTEPS; k++) {
             mma_bf16(d, ab + ((a0 + k * as) >> 4), bb + ((b0 + k * bs) >> 4), idesc, acc);
             acc = 1;
         }
@@ -147,8 +147,8 @@ struct Tables {
 
 // W of the tile as a table [TMAX][LDX], row t: W(t, j), zero above the diagonal; tb.ab[t] = A_t, B_t;
 // tb.wS[j] = theta_j h(j, L-1); tb.tot = A_L, B_L, H_L; tb.wM = W(L-1, .). One thread per column j, the
-// recurrence runs over t: h' = eta_t h, Om' = r_t Om + h'. (One row per thread, unrolled, was 500
-// instructions that every warp fetched once per tile: 2.5k cycles against 1k here.)
+// recurrence runs over t: h' = eta_t h, Om' = r_t Om + h'. With one row per thread (63 unrolled steps in
+// every warp) this stage took the MMA-issuing warp, which the others wait for, 4.6k cycles a tile; 2.8k so.
 template <bool HAS_S>
 __device__ __forceinline__ void decay_table(Tables& tb, float* Wt, int tid, int L)
 {
@@ -188,110 +188,6 @@ __device__ __forceinline__ void decay_row(const Tables& tb, const float* Wt, int
     }
     au = u < 0 ? 1.f : ab.x;
     bu = u < 0 ? 0.f : ab.y;
-}
-
-// X <- (I + Lo)^{-1} X and X <- (I + Lo)^{-T} X for the strictly lower triangular Lo [n16*16 rows],
-// X 64 columns, both fp32 with leading dimension LDX. Blocked by 16 rows: the diagonal block by
-// substitution (one thread per column), the rest as rank-16 updates over all threads.
-__device__ __forceinline__ void diag16(const float* __restrict__ Lo, float* X, int r0, int c)
-{
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) x[i] = X[(r0 + i) * LDX + c];
-#pragma unroll
-    for (int i = 1; i < 16; i++) {
-        const float* row = Lo + (r0 + i) * LDX + r0;
-        float s[4] = {0.f, 0.f, 0.f, 0.f};            // four sums: only the last term waits for row i - 1
-#pragma unroll
-        for (int j4 = 0; j4 < i; j4 += 4) {
-            const float4 l = *reinterpret_cast<const float4*>(row + j4);
-            s[0] = fmaf(l.x, x[j4], s[0]);
-            if (j4 + 1 < i) s[1] = fmaf(l.y, x[j4 + 1], s[1]);
-            if (j4 + 2 < i) s[2] = fmaf(l.z, x[j4 + 2], s[2]);
-            if (j4 + 3 < i) s[3] = fmaf(l.w, x[j4 + 3], s[3]);
-        }
-        x[i] -= (s[0] + s[1]) + (s[2] + s[3]);
-    }
-#pragma unroll
-    for (int i = 1; i < 16; i++) X[(r0 + i) * LDX + c] = x[i];
-}
-__device__ __forceinline__ void diag16_t(const float* __restrict__ Lo, float* X, int r0, int c)
-{
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) x[i] = X[(r0 + i) * LDX + c];
-#pragma unroll
-    for (int k = 15; k >= 1; k--) {
-        const float* row = Lo + (r0 + k) * LDX + r0;
-#pragma unroll
-        for (int j4 = 0; j4 < k; j4 += 4) {
-            const float4 l = *reinterpret_cast<const float4*>(row + j4);
-            x[j4] = fmaf(-l.x, x[k], x[j4]);
-            if (j4 + 1 < k) x[j4 + 1] = fmaf(-l.y, x[k], x[j4 + 1]);
-            if (j4 + 2 < k) x[j4 + 2] = fmaf(-l.z, x[k], x[j4 + 2]);
-            if (j4 + 3 < k) x[j4 + 3] = fmaf(-l.w, x[k], x[j4 + 3]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 15; i++) X[(r0 + i) * LDX + c] = x[i];
-}
-__device__ __forceinline__ void solve_lower(const float* __restrict__ Lo, float* X, int n16)
-{
-    const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-    for (int b = 0; b < n16; b++) {
-        if (g == b) diag16(Lo, X, 16 * b, c);
-        __syncthreads();
-        if (b + 1 < n16) {
-            float x[16];
-#pragma unroll
-            for (int k = 0; k < 16; k++) x[k] = X[(16 * b + k) * LDX + c];
-            for (int i0 = 16 * (b + 1) + 4 * g; i0 < 16 * n16; i0 += 16) {
-                float s[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    float acc = X[(i0 + i) * LDX + c];
-                    const float* row = Lo + (i0 + i) * LDX + 16 * b;
-#pragma unroll
-                    for (int k4 = 0; k4 < 16; k4 += 4) {
-                        const float4 l = *reinterpret_cast<const float4*>(row + k4);
-                        acc = fmaf(-l.x, x[k4], acc); acc = fmaf(-l.y, x[k4 + 1], acc);
-                        acc = fmaf(-l.z, x[k4 + 2], acc); acc = fmaf(-l.w, x[k4 + 3], acc);
-                    }
-                    s[i] = acc;
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) X[(i0 + i) * LDX + c] = s[i];
-            }
-            __syncthreads();
-        }
-    }
-}
-__device__ __forceinline__ void solve_lower_t(const float* __restrict__ Lo, float* X, int n16)
-{
-    const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
-    for (int b = n16 - 1; b >= 0; b--) {
-        if (g == b) diag16_t(Lo, X, 16 * b, c);
-        __syncthreads();
-        if (b > 0) {
-            float x[16];
-#pragma unroll
-            for (int k = 0; k < 16; k++) x[k] = X[(16 * b + k) * LDX + c];
-            for (int i0 = 4 * g; i0 < 16 * b; i0 += 16) {
-                float s[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) s[i] = X[(i0 + i) * LDX + c];
-#pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const float4 l = *reinterpret_cast<const float4*>(Lo + (16 * b + k) * LDX + i0);
-                    s[0] = fmaf(-l.x, x[k], s[0]); s[1] = fmaf(-l.y, x[k], s[1]);
-                    s[2] = fmaf(-l.z, x[k], s[2]); s[3] = fmaf(-l.w, x[k], s[3]);
-                }
-#pragma unroll
-                for (int i = 0; i < 4; i++) X[(i0 + i) * LDX + c] = s[i];
-            }
-            __syncthreads();
-        }
-    }
 }
 
 __device__ __forceinline__ void ld32(float (&v)[32], const float* __restrict__ p, bool ok)
@@ -381,16 +277,16 @@ constexpr int F_KQ = 0, F_MS = 49152, F_WP = 98304, F_E = 122880, F_EW = 147456,
 constexpr int F_TAB = F_X + TMAX * LDX * 4;
 constexpr int FWD_SMEM = F_TAB + (int)sizeof(Tables);
 
-// T tokens per tile. SOLVE: exact rule, else the tile is one frozen chunk.
+// T tokens per tile = per frozen chunk.
 // States are stored at every tile start and after the last token.
-template <int RULE, bool SOLVE>
+template <int RULE>
 __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
 {
     constexpr bool HAS_S = (RULE == RULE_TITANS);
     extern __shared__ __align__(1024) unsigned char sm[];
     Tables& tb = *reinterpret_cast<Tables*>(sm + F_TAB);
     float* Xb = reinterpret_cast<float*>(sm + F_X);      // right-hand side, then E, fp32
-    float* Lb = reinterpret_cast<float*>(sm + F_E);      // Lx, fp32, until the solve is over
+    float* Wt = reinterpret_cast<float*>(sm + F_E);      // table of W until the errors take its place
     const int tid = threadIdx.x, warp = uniform_warp();
     const int R = (warp & 3) * 32 + (tid & 31), hf = warp >> 2;     // TMEM lane, column half
     const int dt = tid - 160;                                       // columns of the decay table: warps 5 to 7
@@ -455,16 +351,15 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<false, false>(tm, kq, 16384, 128, ms, 16384, 128, HAS_S ? 128 : 64, 4);     // K,Q x M0,S0
-            mma6<false, false>(tm + 128, kq, 16384, 128, kq, 16384, 128, 64, 4);             // K,Q x K
+            mma6<false, false>(tm, kq, 16384, 128, ms, 16384, 128, HAS_S ? 128 : 64);     // K,Q x M0,S0
+            mma6<false, false>(tm + 128, kq, 16384, 128, kq, 16384, 128, 64);             // K,Q x K
             mma_commit(smem_u32(&tb.bar[0]));
         }
         float w[32], au, bu;
-        const int u = !krow ? tr : SOLVE ? tr - 1 : -1;
-        decay_table<HAS_S>(tb, Lb, dt, L);           // Lb is free until the scores are in
+        const int u = krow ? -1 : tr;
+        decay_table<HAS_S>(tb, Wt, dt, L);
         __syncthreads();
-        decay_row(tb, Lb, u, hf, w, au, bu);
-        __syncthreads();
+        decay_row(tb, Wt, u, hf, w, au, bu);
         wait(0);
         float acc[32], p[32];
         tload(acc, trow);
@@ -483,19 +378,13 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
                 acc[4 * i] -= v4.x; acc[4 * i + 1] -= v4.y; acc[4 * i + 2] -= v4.z; acc[4 * i + 3] -= v4.w;
             }
             st32(Xb + tr * LDX + hf * 32, acc);
-            if (SOLVE) {
-#pragma unroll
-                for (int i = 0; i < 32; i++) p[i] *= w[i];
-                st32(Lb + tr * LDX + hf * 32, p);
-            }
         } else {
 #pragma unroll
             for (int i = 0; i < 32; i++) p[i] *= -w[i];
             store32(sm + F_WP, 64, 8192, tr, hf * 4, p);
         }
-        if (c + 1 < ntile) fetch(c + 1);         // lands under the solve and the products
+        if (c + 1 < ntile) fetch(c + 1);         // lands under the products
         __syncthreads();
-        if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
         // E and its tile-end weighted copies as planes
 #pragma unroll 1
         for (int i = 0; i < 2; i++) {
@@ -516,9 +405,9 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<true, true>(tm + 256, ew, 16384, 64, kq, 16384, 128, 64, 4);              // [Ew Es]^T K
+            mma6<true, true>(tm + 256, ew, 16384, 64, kq, 16384, 128, 64);              // [Ew Es]^T K
             mma_commit(smem_u32(&tb.bar[1]));
-            mma6<false, true>(tm + 192, wp - 1024, 8192, 64, ep, 8192, 64, 64, 4);         // rows 64..127: -(W o P) E
+            mma6<false, true>(tm + 192, wp - 1024, 8192, 64, ep, 8192, 64, 64);         // rows 64..127: -(W o P) E
             mma_commit(smem_u32(&tb.bar[2]));
         }
         // tile-end states while the outputs' product runs (the partner row is read before anyone
@@ -571,17 +460,14 @@ constexpr int B_KQ = 0, B_YF = 49152, B_WZ = 98304, B_X = 147456, B_E = 196608;
 constexpr int B_TAB = B_E + 24576;
 constexpr int BWD_SMEM = B_TAB + (int)sizeof(Tables);
 
-// mstep: floats between the stored states of consecutive tile starts. SDER (exact rule on a full M
-// trajectory, no S stored): S at a tile start is M_t - (1 - alpha_{t-1}) M_{t-1}, and at the first token
-// (M_1 - r_0 M_0 + theta_0 e_0 k_0^T) / eta_0.
-template <int RULE, bool SOLVE, bool SDER>
-__global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long long mstep)
+// Chunk-boundary states are DD floats apart.
+template <int RULE>
+__global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
 {
     constexpr bool HAS_S = (RULE == RULE_TITANS);
     extern __shared__ __align__(1024) unsigned char sm[];
     Tables& tb = *reinterpret_cast<Tables*>(sm + B_TAB);
     float* Xb = reinterpret_cast<float*>(sm + B_WZ);                  // right-hand sides, fp32
-    float* Lb = reinterpret_cast<float*>(sm + B_WZ + TMAX * LDX * 4);     // Lx, fp32
     float* Ob = Xb + 2 * TMAX * LDX;                                  // dK and dQ on their way out, fp32
     float* Sd = reinterpret_cast<float*>(sm + B_X);                   // scan buffers X -> Xd, and Xs
     float* Ss = reinterpret_cast<float*>(sm + B_X + 17408);
@@ -596,7 +482,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
     const size_t so = (size_t)b * a.seq_len * D, go = (size_t)b * a.seq_len;
     const size_t su = so + un.cc * 8;
     const float* mtraj = a.m_traj + (size_t)b * a.traj_stride;
-    const float* straj = (HAS_S && !SDER) ? a.s_traj + (size_t)b * a.traj_stride : nullptr;
+    const float* straj = HAS_S ? a.s_traj + (size_t)b * a.traj_stride : nullptr;
     const int n = a.t_end - a.t_start;
     const int ntile = (n + T - 1) / T;
 
@@ -620,42 +506,31 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         ld32(g, seed + (size_t)b * DD + tr * D + hf * 32, (HAS_S || krow) && seed != nullptr);
     }
 
+    float gal = 0.f, gth = 0.f, get = 0.f;             // gates of the tile to come, one token per thread
+    auto fetch_gates = [&](int c) {
+        const int t0 = a.t_start + c * T, L = min(T, n - c * T);
+        const bool in = tid < L;
+        gal = in ? a.alpha[go + t0 + tid] : 0.f;
+        gth = in ? a.theta[go + t0 + tid] : 0.f;
+        get = (in && HAS_S) ? a.eta[go + t0 + tid] : 0.f;
+    };
+    if (tid < TMAX) fetch_gates(ntile - 1);
+
     for (int c = ntile - 1; c >= 0; c--) {
         const int t0 = a.t_start + c * T, L = min(T, n - c * T);
-        const bool ok = tr < L;
         auto state_unit = [&](float (&x3)[8], int i) {   // unit i of M0 (0, 1) or S0 (2, 3)
-            const float* mp = mtraj + (size_t)c * mstep;
+            const float* mp = mtraj + (size_t)c * DD;
             const int r = un.row(i & 1), ofs = r * D + un.cc * 8;
             if (i < 2) ld8(x3, mp + ofs);
-            else if (HAS_S && !SDER) ld8(x3, straj + (size_t)c * mstep + ofs);
-            else if (SDER) {
-                const float* m1 = (c > 0) ? mp : mp + DD;
-                const float* m0 = (c > 0) ? mp - DD : mp;
-                const int ta = (c > 0) ? t0 - 1 : t0;
-                const float rr = 1.0f - a.alpha[go + ta];
-                float y3[8];
-                ld8(x3, m1 + ofs);
-                ld8(y3, m0 + ofs);
-#pragma unroll
-                for (int j = 0; j < 8; j++) x3[j] = fmaf(-rr, y3[j], x3[j]);
-                if (c == 0) {
-                    const float* k0 = a.k + so + (size_t)t0 * D;
-                    float e = -a.v[so + (size_t)t0 * D + r];
-#pragma unroll 4
-                    for (int j = 0; j < D; j++) e = fmaf(m0[r * D + j], k0[j], e);
-                    const float te = a.theta[go + t0] * e, et = a.eta[go + t0];
-                    const float inv = et > 1e-30f ? 1.0f / et : 0.f;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) x3[j] = fmaf(te, k0[un.cc * 8 + j], x3[j]) * inv;
-                }
-            } else {
+            else if (HAS_S) ld8(x3, straj + (size_t)c * DD + ofs);
+            else {
 #pragma unroll
                 for (int j = 0; j < 8; j++) x3[j] = 0.f;
             }
         };
         // ── stage 1: operands; K K^T | Q K^T and K,Q x M0,S0 ──
-        // The four units of each matrix go round one loop, the next unit's loads in flight: straight-line
-        // code is fetched once per tile by every warp and was bound by that (8k cycles against 4k).
+        // The four units of each matrix go round one loop with the next unit's loads in flight (as fast as
+        // straight-line code with all 24 loads at once, 8k cycles a tile, and a third of its size).
         {
             float x[8], y[8], x3[8];
             auto get = [&](int i) {                  // K, V, M0 rows, then Q, dY, S0 rows
@@ -682,27 +557,25 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
             }
         }
         if (tid < TMAX) {
-            const bool in = tid < L;
-            tb.gt[tid] = make_float4(in ? 1.0f - a.alpha[go + t0 + tid] : 1.f, (in && HAS_S) ? a.eta[go + t0 + tid] : 0.f,
-                                     in ? a.theta[go + t0 + tid] : 0.f, 0.f);
+            tb.gt[tid] = make_float4(1.0f - gal, get, gth, 0.f);
+            if (c > 0) fetch_gates(c - 1);
         }
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<false, false>(tm, kq, 16384, 128, kq, 16384, 128, 64, 4);
-            mma6<false, false>(tm + 64, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);
+            mma6<false, false>(tm, kq, 16384, 128, kq, 16384, 128, 64);
+            mma6<false, false>(tm + 64, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64);
             mma_commit(smem_u32(&tb.bar[0]));
         }
         if (c > 0 && tid < 4) {                       // the next tile's streams, while this one is worked on
             const float* nx = (tid == 0 ? a.k : tid == 1 ? a.q : tid == 2 ? a.v : a.d_y) + so + (size_t)(t0 - T) * D;
             l2_prefetch(nx, (unsigned)T * D * 4);
         } else if (c > 0 && tid < 6) {
-            if (tid == 4) l2_prefetch(mtraj + (size_t)(c - 1) * mstep, DD * 4);
-            else if (straj != nullptr) l2_prefetch(straj + (size_t)(c - 1) * mstep, DD * 4);
-            else if (SDER && c > 1) l2_prefetch(mtraj + (size_t)(c - 1) * mstep - DD, DD * 4);
+            if (tid == 4) l2_prefetch(mtraj + (size_t)(c - 1) * DD, DD * 4);
+            else if (HAS_S) l2_prefetch(straj + (size_t)(c - 1) * DD, DD * 4);
         }
         float w[32], p[32], au, bu;
-        const int u = !krow ? tr : SOLVE ? tr - 1 : -1;
+        const int u = krow ? -1 : tr;
         float dots[2] = {0.f, 0.f};                   // <M0, G_M> or <S0, G_S>; <S0, G_M>
 #pragma unroll
         for (int c8 = 0; c8 < 4; c8++) {
@@ -742,11 +615,6 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
                     for (int i = 0; i < 32; i++) acc[i] = fmaf(bu, s[i], acc[i]);
                 }
                 st32(Xb + tr * LDX + hf * 32, acc);
-                if (SOLVE) {
-#pragma unroll
-                    for (int i = 0; i < 32; i++) acc[i] = w[i] * p[i];
-                    st32(Lb + tr * LDX + hf * 32, acc);
-                }
             } else {
                 float zm = 0.f, zs = 0.f, y[32];
 #pragma unroll
@@ -762,7 +630,6 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
             }
         }
         __syncthreads();
-        if (SOLVE) solve_lower(Lb, Xb, (L + 15) >> 4);
         // ── stage 2: E planes, W o P, G planes; right-hand side of F, E x G ──
 #pragma unroll 1
         for (int i = 0; i < 2; i++) {
@@ -780,11 +647,11 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<false, false>(tm, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64, 4);              // K G^T
-            mma6<true, true>(tm + 128, wz + 24576, 8192, 64, yf + 1024, 16384, 128, 64, 4);           // (W o P)^T dY
+            mma6<false, false>(tm, kq, 16384, 128, xx, 16384, 128, HAS_S ? 128 : 64);              // K G^T
+            mma6<true, true>(tm + 128, wz + 24576, 8192, 64, yf + 1024, 16384, 128, 64);           // (W o P)^T dY
             mma_commit(smem_u32(&tb.bar[0]));
-            mma6<false, true>(tm + 192, ep, 8192, 64, xx, 16384, 128, 64, 4);                         // E G_M
-            if (HAS_S) mma6<false, true>(tm + 256, ep, 8192, 64, xx + 1024, 16384, 128, 64, 4);       // E G_S
+            mma6<false, true>(tm + 192, ep, 8192, 64, xx, 16384, 128, 64);                         // E G_M
+            if (HAS_S) mma6<false, true>(tm + 256, ep, 8192, 64, xx + 1024, 16384, 128, 64);       // E G_S
             mma_commit(smem_u32(&tb.bar[1]));
         }
         wait(0);
@@ -802,14 +669,8 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
                 for (int i = 0; i < 32; i++) dx[i] = fmaf(-wsv, s[i], dx[i]);
             }
             st32(Xb + tr * LDX + hf * 32, dx);
-            if (SOLVE) {
-#pragma unroll
-                for (int i = 0; i < 32; i++) s[i] = w[i] * p[i];
-                st32(Lb + tr * LDX + hf * 32, s);
-            }
         }
         __syncthreads();
-        if (SOLVE) solve_lower_t(Lb, Xb, (L + 15) >> 4);
         wait(1);
         if (krow) {
             const float wm = tb.wM[tr], wsv = HAS_S ? tb.wS[tr] : 0.f;
@@ -861,10 +722,10 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<false, false>(tm, yf, 16384, 128, ep, 8192, 64, 64, 4);                       // F,dY x E
+            mma6<false, false>(tm, yf, 16384, 128, ep, 8192, 64, 64);                       // F,dY x E
             mma_commit(smem_u32(&tb.bar[0]));
-            mma6<false, true>(tm + 64, yf, 16384, 128, xx, 16384, 128, 64, 4);                 // F,dY x M0
-            if (HAS_S) mma6<false, true>(tm + 128, yf, 16384, 128, xx + 1024, 16384, 128, 64, 4);   // F,dY x S0
+            mma6<false, true>(tm + 64, yf, 16384, 128, xx, 16384, 128, 64);                 // F,dY x M0
+            if (HAS_S) mma6<false, true>(tm + 128, yf, 16384, 128, xx + 1024, 16384, 128, 64);   // F,dY x S0
             mma_commit(smem_u32(&tb.bar[1]));
         }
         wait(0);
@@ -873,7 +734,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
             tload(s, trow);                            // N row (krow) or R row
 #pragma unroll
             for (int i = 0; i < 32; i++) { p[i] *= s[i]; s[i] *= -w[i]; }
-            store32(sm + B_WZ, 128, 16384, R, hf * 4, s);
+            if (!krow) store32(sm + B_WZ, 128, 16384, R, hf * 4, s);
             wait(1);
             if (!krow) {
                 // every read of the state planes by the tensor cores is over: the scan buffers take their place
@@ -885,20 +746,6 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
             float s2[32];
             tload(s, trow + 64);
             if (HAS_S) tload(s2, trow + 128);
-            if (SOLVE && krow) {
-                float zkm = 0.f, zks = 0.f;
-#pragma unroll
-                for (int c8 = 0; c8 < 4; c8++) {
-                    float kk[8];
-                    load8(kk, kqp, 128, 16384, R, hf * 4 + c8);
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        zkm = fmaf(kk[i], s[8 * c8 + i], zkm);
-                        if (HAS_S) zks = fmaf(kk[i], s2[8 * c8 + i], zks);
-                    }
-                }
-                tb.part[0][hf * 64 + tr] = zkm; tb.part[1][hf * 64 + tr] = zks;
-            }
 #pragma unroll
             for (int i = 0; i < 32; i++) {
                 dx[i] = krow ? fmaf(au, s[i], dx[i]) : au * s[i];
@@ -906,21 +753,12 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
             }
         }
         publish();
-        // ── stage 4: (W o R, Z) x K and transposes; gate scans under them ──
+        // ── stage 4: -(W o R) K and -(W o R)^T Q; gate scans under them ──
         if (warp == 4 && elect_one()) {                // warps 0 to 2 have the scans to do
             fence_after_sync();
-            mma6<false, true>(tm + 192, wz, 16384, 128, kq, 16384, 128, 64, 4);        // rows: Z K | -(W o R) K
-            mma6<true, true>(tm + 256, wz, 16384, 128, kq, 16384, 128, 64, 8);         // Z^T K - (W o R)^T Q
+            mma6<false, true>(tm + 192, wz, 16384, 128, kq, 16384, 128, 64);        // rows 64..127: -(W o R) K
+            mma6<true, true>(tm + 256, wz + 1024, 16384, 128, kq + 1024, 16384, 128, 64);  // -(W o R)^T Q
             mma_commit(smem_u32(&tb.bar[0]));
-        }
-        if (SOLVE) {
-            if (krow && u >= 0 && ok) {
-#pragma unroll
-                for (int i = 0; i < 32; i++) Sd[u * LDS + hf * 32 + i] += p[i];
-                // the M0 and S0 columns take the error's share too
-                Sd[u * LDS + 64 + hf] += tb.part[hf][tr] + tb.part[hf][64 + tr];
-            }
-            __syncthreads();
         }
         if (tid < 66) {                                // decayed scans, one column per thread
             const int j = tid;
@@ -1002,14 +840,9 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         wait(0);
         {
             float s[32];
-            tload(s, trow + 192);
+            tload(s, trow + (krow ? 256 : 192));
 #pragma unroll
             for (int i = 0; i < 32; i++) dx[i] += s[i];
-            if (krow) {
-                tload(s, trow + 256);
-#pragma unroll
-                for (int i = 0; i < 32; i++) dx[i] += s[i];
-            }
         }
         __syncthreads();                               // the scan buffers have been read
         // ── stage 5: carry. [diag(a) F ; diag(A) dY | diag(b) F ; diag(B) dY]^T [K ; Q] ──
@@ -1029,7 +862,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         publish();
         if (warp == 0 && elect_one()) {
             fence_after_sync();
-            mma6<true, true>(tm + 320, wz, 32768, 128, kq, 16384, 128, 64, 8);
+            mma6<true, true, 8>(tm + 320, wz, 32768, 128, kq, 16384, 128, 64);
             mma_commit(smem_u32(&tb.bar[0]));
         }
         const float At = tb.tot[0], Bt = tb.tot[1], Ht = tb.tot[2];
@@ -1053,7 +886,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T, long 
         st32(Ob + R * LDX + hf * 32, dx);
         fence_before_sync();
         __syncthreads();
-#pragma unroll
+#pragma unroll 1
         for (int i = 0; i < 4; i++) {
             const int r = un.row(i & 1);
             if (r < L) copy8((i < 2 ? a.d_k : a.d_q) + su + (size_t)(t0 + r) * D, Ob + un.row(i) * LDX + un.cc * 8);

@@ -7,10 +7,8 @@
 namespace nlh {
 namespace mtc {
 
-// a.interval = tile length = distance of the stored states
 bool forward(int rule, const FwdArgs& a, cudaStream_t st);
-// T = tile length, mstep = floats between the stored states of consecutive tile starts
-bool backward(int rule, const BwdArgs& a, int T, long long mstep, cudaStream_t st);
+bool backward(int rule, const BwdArgs& a, cudaStream_t st);
 int timeout_flag();
 
 }  // namespace mtc

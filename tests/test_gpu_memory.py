@@ -155,6 +155,28 @@ def test_chunk_matrix_form_matches_per_token_kernels(D, orc):
         assert rel_err(_np(res[0][key]), _np(res[1][key])) <= REL, key
 
 
+@pytest.mark.parametrize("rule", ["titans", "delta"])
+@pytest.mark.parametrize("s,chunk", [(1, 64), (16, 16), (33, 16), (17, 17), (63, 64), (64, 64), (65, 64), (100, 48), (130, 64)])
+def test_chunk_tiles_at_their_edges(D, orc, rule, s, chunk):
+    """Frozen rule in matrix form (head_dim 64, tiles of 16 to 64 tokens): full, ragged and single-token last
+    tiles against the oracle, and a second pass gives the same bits."""
+    p = make_problem(orc, 3, s, 64, 5200 + s + chunk, "rand")
+    w = oracle_chunkwise(orc, rule, p, chunk)
+    t = to_dev(p)
+    r = 1 if rule == "titans" else 0
+    eta, s0 = (t["eta"], t["s0"]) if r else (None, None)
+    runs = []
+    for _ in range(2):
+        mc, sc, y = D.rule_forward(r, t["k"], t["v"], t["q"], t["alpha"], t["theta"], eta, t["m0"], s0, chunk, chunk)
+        g = D.rule_backward(r, t["k"], t["v"], t["q"], t["alpha"], t["theta"], eta, mc, sc, t["dy"], chunk, chunk)
+        runs.append({n: _np(x) for n, x in dict(g, y=y, mc=mc, sc=sc).items() if x is not None})
+    for key in runs[0]:
+        assert np.array_equal(runs[0][key], runs[1][key]), key
+    assert rel_err(runs[0]["y"], w["y"]) <= REL
+    assert rel_err(runs[0]["mc"], w["m_chunk_states"]) <= REL
+    _check_bwd(g, w, ["d_k", "d_v", "d_q", "d_alpha", "d_theta"] + (["d_eta"] if r else []), tol_abs=1e-3)
+
+
 def test_chunk1_matches_per_token_kernel(D, orc):
     # core/src/gpu_forward.rs:4193-4300: C=1 chunkwise == per-token kernel (<1e-5)
     p = make_problem(orc, 2, 16, 64, 1200, "const")
