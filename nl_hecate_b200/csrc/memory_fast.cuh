@@ -737,9 +737,10 @@ __global__ void __launch_bounds__(FastGeom<D, SPLIT>::NT, (D == 64 && !FROZEN) ?
                 for (int i = lane; i < ROWS; i += 32) s += scp[(which * TB + tl) * ROWS + i];
                 s = warp_sum(s);
                 if (lane == 0) {
-                    float* dst = which == 0 ? dalpha + tt0 + tl : which == 1 ? dtheta + tt0 + tl : deta + tt0 + tl;
-                    const float val = which == 2 ? s : -s;
-                    if (SPLIT > 1) atomicAdd(dst, val); else *dst = val;
+                    if (SPLIT > 1) atomicAdd(which == 0 ? dalpha + tt0 + tl : which == 1 ? dtheta + tt0 + tl : deta + tt0 + tl, which == 2 ? s : -s);
+                    else if (which == 0) dalpha[tt0 + tl] = -s;
+                    else if (which == 1) dtheta[tt0 + tl] = -s;
+                    else deta[tt0 + tl] = s;
                 }
             }
             // the next tile's first-token barrier orders these reads before pq/pk/scp are rewritten
