@@ -33,7 +33,8 @@
 // tile's stages: tensor products (55 cycles per 128x64x16 plane product, the A operand is read from
 // shared memory for each; 22k of a backward tile's cycles), loads and the conversion of every intermediate
 // into planes with two warps per scheduler. The stage times are the same with 4 problems as with 128, so
-// neither memory nor the other SMs bound them.
+// neither memory nor the other SMs bound them. Forward and backward, 128 problems x 2048 tokens, chunk 64:
+// 1802 us with fp32 FMA contractions in shared memory, 1177 us so (Delta, 24 x 1000, chunk 48: 903 -> 633).
 //
 // Shared-memory matrices: element (row, col) of an R-row plane at (col/8)*(R*16) + row*16 + (col%8)*2,
 // the canonical no-swizzle core-matrix layout with the 8-column chunk outermost. The same bytes serve

@@ -90,7 +90,7 @@ class FlatAdamW:
             self._row_busy[r] = False
         row = self._desc_rows[r]
         t = np.maximum(np.asarray(steps, dtype=np.int64), 1)
-        if (t == t[0]).all():                    # one count for all tensors: one power per moment
+        if t.size and (t == t[0]).all():                    # one count for all tensors: one power per moment
             t = t[:1]
         row["bc1_inv"] = 1.0 / (1.0 - self.beta1 ** t.astype(np.float64))
         row["bc2_inv"] = 1.0 / (1.0 - self.beta2 ** t.astype(np.float64))
