@@ -1060,7 +1060,8 @@ class StackedMAG:
         clip, AdamW, weight tying): removes the per-launch host cost, which dominates when the
         per-rank batch is small. The first call runs two eager steps (sizes every allocation and
         the library workspace) and captures; later calls copy the inputs into static buffers and
-        replay. Shapes must not change between calls."""
+        replay. Shapes must not change between calls. The inputs have been read when the call returns:
+        a loader may refill its (pinned) buffers then. The step itself is only queued."""
         if getattr(self, "_graph", None) is None:
             self._static_tok = tokens.clone()
             self._static_tgt = targets.clone()
@@ -1081,14 +1082,19 @@ class StackedMAG:
                 self.sync_gradients(process_group, world)
                 self._device_update()
             self._graph.replay()            # capture records only: run the scheduled step now
+            self._inputs_read = torch.cuda.Event()
             return self._static_loss
         self._static_tok.copy_(tokens, non_blocking=True)
         self._static_tgt.copy_(targets, non_blocking=True)
+        self._inputs_read.record()
         # the descriptors go to the device ahead of the replay, stream-ordered: the host does not wait
         # for the previous step and its bookkeeping runs while the GPU is still busy with it
         self._host_schedule()
         self.opt.upload()
         self._graph.replay()
+        # the copies sit behind the previous step: without this wait the caller could overwrite them
+        # unread. The replay is queued already, so the GPU has this step to do meanwhile.
+        self._inputs_read.synchronize()
         return self._static_loss
 
     def n_params(self):

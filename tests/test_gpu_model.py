@@ -145,6 +145,38 @@ def test_graph_replayed_step_matches_eager_steps():
             assert float((a - r).abs().max()) <= 1e-3 * max(float(r.abs().max()), 1e-6)
 
 
+def test_graphed_steps_train_on_the_batch_of_their_call():
+    """Two pinned buffers, refilled in turn as soon as a call returned while the GPU is behind: the
+    weights are those of a run that waits for every step."""
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from nl_hecate_b200.stacked_mag import StackedMAG
+
+    batches = [tuple(t.cpu() for t in _data(4, seed=60 + step)) for step in range(6)]
+
+    def run(wait):
+        model = StackedMAG(_cfg(True), 4, device="cuda", seed=7)
+        model.step_graphed(*_data(4, seed=50))
+        host = [tuple(torch.empty_like(t).pin_memory() for t in batches[0]) for _ in range(2)]
+        torch.cuda.synchronize()
+        if not wait:                                 # some ms of queued work ahead of the steps
+            a = torch.randn(4096, 4096, device="cuda")
+            for _ in range(40):
+                a = (a @ a) * 1e-4
+        for step in range(6):
+            for buf, t in zip(host[step % 2], batches[step]):
+                buf.copy_(t)
+            loss = model.step_graphed(*host[step % 2])
+            if wait:
+                torch.cuda.synchronize()
+        return float(loss), model.opt.w.clone()
+
+    (la, wa), (lb, wb) = run(True), run(False)
+    # a step on another batch moves the loss and the weights far more than the order of atomic adds does
+    assert abs(la - lb) <= 1e-3 * abs(la)
+    assert float((wa - wb).abs().max()) <= 1e-4
+
+
 def test_checkpointed_exact_level_matches_the_stored_trajectory():
     """cfg.exact_checkpoint: level 0 keeps a checkpoint every 8 tokens and recomputes the windows in
     the backward: same loss and gradients as the stored-trajectory pair (both fp32 state; the

@@ -1,0 +1,99 @@
+"""CPU tests of the host path around the kernels: what a call may still read after it has returned,
+which descriptors an optimizer step uses, and what the C-ABI call layer refuses. The GPU is replaced by
+a queue of deferred operations where the order of host and device work matters."""
+import contextlib
+import os
+import sys
+
+import pytest
+import torch
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+
+
+class _Queue:
+    """A stream that runs nothing until someone waits for it: the slowest GPU there can be."""
+
+    def __init__(self):
+        self.ops = []
+
+    def push(self, op):
+        self.ops.append(op)
+        return len(self.ops)
+
+    def drain(self, upto=None):
+        upto = len(self.ops) if upto is None else upto
+        for i in range(upto):
+            if self.ops[i] is not None:
+                op, self.ops[i] = self.ops[i], None
+                op()
+
+
+def _graphed_model(monkeypatch, queue):
+    """StackedMAG with everything but step_graphed itself replaced; replay() notes the static inputs that
+    the step would have trained on."""
+    from nl_hecate_b200.stacked_mag import StackedMAG
+
+    class Event:
+        def __init__(self, *a, **k):
+            self.at = 0
+
+        def record(self, *a):
+            self.at = queue.push(lambda: None)
+
+        def synchronize(self):
+            queue.drain(self.at)
+
+    class Graph:
+        def replay(self):
+            queue.push(lambda: m.trained_on.append((int(m._static_tok.t[0]), int(m._static_tgt.t[0]))))
+
+    class Stream:
+        def wait_stream(self, s):
+            pass
+
+    class Static:
+        def __init__(self, t):
+            self.t = t
+
+        def copy_(self, src, non_blocking=False):
+            queue.push(lambda: self.t.copy_(src))
+
+    nothing = lambda *a, **k: None
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "Stream", Stream)
+    monkeypatch.setattr(torch.cuda, "current_stream", Stream)
+    monkeypatch.setattr(torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "synchronize", nothing)
+    monkeypatch.setattr(torch.cuda, "empty_cache", nothing)
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", Graph)
+    monkeypatch.setattr(torch.cuda, "graph", lambda g: contextlib.nullcontext())
+    m = StackedMAG.__new__(StackedMAG)
+    m.step = m.sync_gradients = m._device_update = m._host_schedule = nothing
+    m.forward_backward = lambda *a: torch.zeros(())
+    m.opt = type("Opt", (), {"upload": nothing})()
+    m.trained_on = []
+    # the first call captures; the static inputs that it clones become deferred buffers
+    inputs = torch.zeros(1), torch.zeros(1)
+    clone = torch.Tensor.clone
+    with monkeypatch.context() as mp:
+        mp.setattr(torch.Tensor, "clone", lambda t: Static(clone(t)))
+        m.step_graphed(*inputs)
+    queue.drain()
+    m.trained_on.clear()
+    return m
+
+
+@pytest.mark.parametrize("buffers", [1, 2])
+def test_graphed_step_has_read_its_inputs_when_it_returns(monkeypatch, buffers):
+    """A loader refills one pinned buffer, or two in turn, as soon as a call returned: every step must
+    train on what the buffers held when it was called."""
+    queue = _Queue()
+    m = _graphed_model(monkeypatch, queue)
+    host = [(torch.zeros(1), torch.zeros(1)) for _ in range(buffers)]
+    for step in range(6):
+        tok, tgt = host[step % buffers]
+        tok.fill_(step), tgt.fill_(100 + step)
+        m.step_graphed(tok, tgt)
+    queue.drain()
+    assert m.trained_on == [(s, 100 + s) for s in range(6)]
