@@ -134,7 +134,11 @@ class _TitansMemory(torch.autograd.Function):
             # the carried memory is updated in place from the last stored state (one strided copy;
             # the kernels have read m0 by then, stream order), no separate m_final tensor
             n, slots, dd = ms.shape
-            D.call("nlh_copy_rows", src=ms[:, -1].data_ptr(), src_stride=slots * dd, dst=carry, rows=n, row_len=dd)
+            if carry.dtype == ms.dtype and carry.shape == (n, dd) and carry.is_contiguous() and carry.device == ms.device:
+                D.call("nlh_copy_rows", src=ms[:, -1].data_ptr(), src_stride=slots * dd, dst=carry, rows=n, row_len=dd)
+                torch.autograd.graph.increment_version(carry)   # written past autograd
+            else:
+                carry.copy_(ms[:, -1])
             return y, None
         m_final = ms[:, -1].clone()
         ctx.mark_non_differentiable(m_final)
@@ -1038,6 +1042,7 @@ class StackedMAG:
             # gpu_stacked_sync_embed_weights: w_embed <- w_unembed^T
             if self.device.type == "cuda":
                 D.call("nlh_transpose", src=self.p["w_unembed"], dst=self.p["w_embed"], rows=cfg.d_model, cols=cfg.vocab)
+                torch.autograd.graph.increment_version(self.p["w_embed"])    # written past autograd
             else:
                 with torch.no_grad():
                     self.p["w_embed"].copy_(self.p["w_unembed"].t())

@@ -97,3 +97,27 @@ def test_graphed_step_has_read_its_inputs_when_it_returns(monkeypatch, buffers):
         m.step_graphed(tok, tgt)
     queue.drain()
     assert m.trained_on == [(s, 100 + s) for s in range(6)]
+
+
+@pytest.mark.parametrize("form", ["plain", "double", "transposed", "per head"])
+def test_carried_memory_takes_every_form_that_copy_takes(monkeypatch, form):
+    """The row-gather kernel writes n x d*d contiguous fp32 values: a carry of another type, stride or
+    shape is copied by torch as before (and refused by it where the shapes do not match)."""
+    from nl_hecate_b200 import stacked_mag as sm
+    n, s, d = 3, 5, 4
+    ms = torch.randn(n, s + 1, d * d)
+    kernel = []
+    monkeypatch.setattr(sm.D, "titans_forward_dd", lambda *a, **k: (ms, None, torch.zeros(n, s, d)))
+    monkeypatch.setattr(sm.D, "call", lambda name, **k: kernel.append((name, k)))
+    ctx = type("Ctx", (), {"save_for_backward": lambda self, *t: None})()
+    carry = {"plain": torch.zeros(n, d * d), "double": torch.zeros(n, d * d, dtype=torch.float64),
+             "transposed": torch.zeros(d * d, n).t(), "per head": torch.zeros(1, n, d * d)}[form]
+    x = torch.zeros(n, s, d)
+    version = carry._version
+    sm._TitansMemory._forward(ctx, x, x, x, x, x, x, ms[:, 0], ms[:, 0], 0, carry)
+    if form == "plain":
+        assert [c[0] for c in kernel] == ["nlh_copy_rows"] and carry._version > version
+    else:
+        assert not kernel and torch.equal(carry.reshape(n, d * d).float(), ms[:, -1])
+    with pytest.raises(RuntimeError):
+        sm._TitansMemory._forward(ctx, x, x, x, x, x, x, ms[:, 0], ms[:, 0], 0, torch.zeros(n - 1, d * d))
