@@ -48,21 +48,16 @@ class FlatAdamW:
         self.chunk_tensor = torch.tensor(ct, dtype=torch.int32, device=dev)
         self.chunk_start = torch.tensor(cs, dtype=torch.int64, device=dev)
         self.chunk_len = torch.tensor(cl, dtype=torch.int32, device=dev)
-        # Per-tensor descriptors of one step. The columns that stay are written once into every row of
-        # the ring. The table travels through a small ring of pinned host rows: prepare() fills the
-        # next one while the GPU may still have to read the previous ones, so the host runs ahead of
-        # the device.
+        # Per-tensor descriptors of one step. The table travels through a small ring of pinned host rows:
+        # prepare() fills the next one while the GPU may still have to read the previous ones, so the
+        # host runs ahead of the device.
         nt = len(self.sizes)
-        base = np.zeros(nt, dtype=_DESC)
-        self._row_decay = [None] * RING
-        for i, (lo, hi) in self.clamp.items():
-            base["clamp_lo"][i], base["clamp_hi"][i], base["has_clamp"][i] = lo, hi, 1
-        pinned = torch.empty(RING, nt * _DESC.itemsize, dtype=torch.uint8)
+        pinned = torch.zeros(RING, nt * _DESC.itemsize, dtype=torch.uint8)
         if dev.type == "cuda":
             pinned = pinned.pin_memory()
         self._desc_ring = pinned
         self._desc_rows = pinned.numpy().view(_DESC)
-        self._desc_rows[:] = base
+        self._row_options = [None] * RING      # the (weight_decay, no_decay, clamp) that a row was filled with
         self._desc_dev = torch.empty(nt * _DESC.itemsize, dtype=torch.uint8, device=dev)
         self._partial = torch.empty(148 * 8, dtype=torch.float32, device=dev)
         self.norm = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -84,22 +79,30 @@ class FlatAdamW:
         """Host part of a step: fill the next row of the descriptor ring (bias corrections from each
         tensor's own 1-based step count, activity, learning-rate scale). The device reads it after
         upload(); a row is rewritten only when the upload that last used it has completed."""
-        r = self._row = (self._row + 1) % RING if self._captured_row is None else self._captured_row
+        nt = len(self.sizes)
+        if nt and type(steps) is list and len(steps) >= nt and steps[:nt].count(steps[0]) == nt:   # one count for all
+            t = [max(int(steps[0]), 1)]
+        else:
+            t = [max(int(steps[i]), 1) for i in range(nt)]
+        bc = {x: (1.0 / (1.0 - self.beta1 ** x), 1.0 / (1.0 - self.beta2 ** x)) for x in set(t)}
+        act = [1] if active is None else [bool(active[i]) for i in range(nt)]
+        r = (self._row + 1) % RING if self._captured_row is None else self._captured_row
         if self._row_busy[r]:
             self._uploaded[r].synchronize()
             self._row_busy[r] = False
         row = self._desc_rows[r]
-        t = np.maximum(np.asarray(steps, dtype=np.int64), 1)
-        if t.size and (t == t[0]).all():                    # one count for all tensors: one power per moment
-            t = t[:1]
-        row["bc1_inv"] = 1.0 / (1.0 - self.beta1 ** t.astype(np.float64))
-        row["bc2_inv"] = 1.0 / (1.0 - self.beta2 ** t.astype(np.float64))
+        row["bc1_inv"] = [bc[x][0] for x in t]
+        row["bc2_inv"] = [bc[x][1] for x in t]
         row["lr_scale"] = lr_scale
-        if self.weight_decay != self._row_decay[r]:
-            row["weight_decay"] = self.weight_decay
-            row["weight_decay"][list(self.no_decay)] = 0.0
-            self._row_decay[r] = self.weight_decay
-        row["active"] = True if active is None else np.asarray(active, dtype=bool)
+        row["active"] = act
+        options = (self.weight_decay, self.no_decay, self.clamp)
+        if options != self._row_options[r]:     # these rarely change: compared, not rewritten, each step
+            row["weight_decay"] = [0.0 if i in self.no_decay else self.weight_decay for i in range(nt)]
+            row["clamp_lo"] = [self.clamp[i][0] if i in self.clamp else 0.0 for i in range(nt)]
+            row["clamp_hi"] = [self.clamp[i][1] if i in self.clamp else 0.0 for i in range(nt)]
+            row["has_clamp"] = [i in self.clamp for i in range(nt)]
+            self._row_options[r] = (self.weight_decay, set(self.no_decay), dict(self.clamp))
+        self._row = r
         self._prepared = True
 
     def upload(self):

@@ -121,3 +121,43 @@ def test_carried_memory_takes_every_form_that_copy_takes(monkeypatch, form):
         assert not kernel and torch.equal(carry.reshape(n, d * d).float(), ms[:, -1])
     with pytest.raises(RuntimeError):
         sm._TitansMemory._forward(ctx, x, x, x, x, x, x, ms[:, 0], ms[:, 0], 0, torch.zeros(n - 1, d * d))
+
+
+def _rows(opt):
+    return opt._desc_rows[opt._row]
+
+
+def test_prepare_reads_clamp_and_no_decay_at_every_step():
+    """Both are public attributes: a change between two steps counts from the next step on, in every row of
+    the descriptor ring; an index that names no tensor names none."""
+    from nl_hecate_b200.optimizer import RING, FlatAdamW
+    opt = FlatAdamW([8, 8, 8], device="cpu", weight_decay=0.1, clamp={1: (-1.0, 1.0)}, no_decay=[0, -1, 7])
+    for i in range(2 * RING + 1):
+        if i == RING - 1:
+            opt.clamp[2] = (-2.0, 3.0)
+            del opt.clamp[1]
+            opt.no_decay = {2}
+        opt.prepare([1, 1, 1])
+        r = _rows(opt)
+        changed = i >= RING - 1
+        assert list(r["has_clamp"]) == ([0, 0, 1] if changed else [0, 1, 0])
+        assert list(r["clamp_lo"]) == ([0, 0, -2] if changed else [0, -1, 0])
+        assert list(r["clamp_hi"]) == ([0, 0, 3] if changed else [0, 1, 0])
+        assert [x > 0 for x in r["weight_decay"]] == ([True, True, False] if changed else [False, True, True])
+
+
+def test_prepare_takes_one_step_count_and_flag_per_tensor():
+    """Anything that can be indexed by tensor, more entries than tensors among it; too few are refused."""
+    from nl_hecate_b200.optimizer import FlatAdamW
+    opt = FlatAdamW([8, 8, 8], device="cpu")
+    want = [1.0 / (1.0 - 0.9 ** t) for t in (1, 2, 3)]
+    for steps in ([1, 2, 3], (0, 2, 3), [1, 2, 3, 9], {0: 1, 1: 2, 2: 3}, torch.tensor([1, 2, 3]), [1.5, 2.5, 3.0]):
+        opt.prepare(steps, [1, 0, 2, 0])
+        assert _rows(opt)["bc1_inv"].tolist() == pytest.approx(want, rel=1e-7)
+        assert list(_rows(opt)["active"]) == [1, 0, 1]
+    for steps, active in (([1], None), ([], None), ([1, 2], None), ([1, 2, 3], [True]), ([1, 2, 3], True)):
+        with pytest.raises((IndexError, TypeError)):
+            opt.prepare(steps, active)
+    opt.beta1 = 1.0
+    with pytest.raises(ZeroDivisionError):
+        opt.prepare([1, 2, 3])
