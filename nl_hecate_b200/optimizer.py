@@ -69,7 +69,7 @@ class FlatAdamW:
         self._row_busy = [False] * RING
         self._row = 0
         self._captured_row = None      # set when a graph captured the upload of a row: that row is then reused
-        self._prepared = False
+        self._on_device = False        # the caller uploaded the prepared row itself
 
     def view(self, arena: torch.Tensor, i: int) -> torch.Tensor:
         o, n = self.slices[i]
@@ -78,7 +78,9 @@ class FlatAdamW:
     def prepare(self, steps, active=None, lr_scale=1.0):
         """Host part of a step: fill the next row of the descriptor ring (bias corrections from each
         tensor's own 1-based step count, activity, learning-rate scale). The device reads it after
-        upload(); a row is rewritten only when the upload that last used it has completed."""
+        launch() or upload(); a row is rewritten only when the upload that last used it has completed. A
+        graph that captured launch() without an upload() before it reads the same row at every replay:
+        its caller waits for a replay before it prepares the next one."""
         nt = len(self.sizes)
         if nt and type(steps) is list and len(steps) >= nt and steps[:nt].count(steps[0]) == nt:   # one count for all
             t = [max(int(steps[0]), 1)]
@@ -103,12 +105,16 @@ class FlatAdamW:
             row["has_clamp"] = [i in self.clamp for i in range(nt)]
             self._row_options[r] = (self.weight_decay, set(self.no_decay), dict(self.clamp))
         self._row = r
-        self._prepared = True
+        self._on_device = False
 
     def upload(self):
-        """Stream-ordered copy of the prepared descriptors to the device. launch() does it itself;
-        a caller that replays a captured launch() calls it before the capture and before every
-        replay, so that the graph holds no copy from a fixed host row."""
+        """Stream-ordered copy of the prepared descriptors to the device, for a caller that replays a
+        captured launch(): with an upload() before the capture and before every replay the graph holds no
+        copy from a fixed host row. launch() uploads by itself what the caller has not."""
+        self._upload()
+        self._on_device = True
+
+    def _upload(self):
         r = self._row
         self._desc_dev.copy_(self._desc_ring[r], non_blocking=True)
         if self._uploaded is None:
@@ -118,14 +124,13 @@ class FlatAdamW:
         else:
             self._uploaded[r].record()
             self._row_busy[r] = True
-        self._prepared = False
 
     def launch(self, lr, max_grad_norm=0.0):
-        """Device part of a step (stream-ordered, capturable in a CUDA graph): upload of descriptors
-        that are not on the device yet, global-norm clip scale, multi-tensor AdamW. Returns the device
-        scalar with the pre-clip gradient norm (valid only when max_grad_norm > 0)."""
-        if self._prepared:
-            self.upload()
+        """Device part of a step (stream-ordered, capturable in a CUDA graph): descriptor upload,
+        global-norm clip scale, multi-tensor AdamW. Returns the device scalar with the pre-clip
+        gradient norm (valid only when max_grad_norm > 0)."""
+        if not self._on_device:
+            self._upload()
         scale_ptr = None
         if max_grad_norm > 0.0:
             call("nlh_arena_grad_norm_clip", g=self.g, n=self.arena_len,

@@ -161,3 +161,93 @@ def test_prepare_takes_one_step_count_and_flag_per_tensor():
     opt.beta1 = 1.0
     with pytest.raises(ZeroDivisionError):
         opt.prepare([1, 2, 3])
+
+
+def _optimizer_on_a_fake_device(monkeypatch):
+    """FlatAdamW whose launches note the descriptors on the device; `captured` collects what a stream capture
+    would record (uploads and launches), to be replayed."""
+    from nl_hecate_b200 import optimizer as om
+    opt = om.FlatAdamW([8, 8], device="cpu")
+    opt.seen = []
+    captured = []
+    state = {"capturing": False}
+    nt, item = len(opt.sizes), om._DESC
+
+    def launch(name, **k):
+        if name == "nlh_adamw_multi_tensor":
+            op = lambda: opt.seen.append(opt._desc_dev.t.numpy().view(item)["active"].tolist())
+            captured.append(op) if state["capturing"] else op()
+
+    class Dev:
+        def __init__(self, t):
+            self.t = t
+
+        def copy_(self, src, non_blocking=False):
+            op = lambda: self.t.copy_(src)
+            captured.append(op) if state["capturing"] else op()
+
+    class Event:
+        def record(self, *a):
+            assert not state["capturing"]
+
+        def synchronize(self):
+            pass
+
+    monkeypatch.setattr(om, "call", launch)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: state["capturing"])
+    opt._desc_dev = Dev(torch.zeros(nt * item.itemsize, dtype=torch.uint8))
+    opt._uploaded = [Event() for _ in range(om.RING)]
+
+    @contextlib.contextmanager
+    def capture():
+        state["capturing"] = True
+        yield
+        state["capturing"] = False
+
+    def replay():
+        for op in captured:
+            op()
+    return opt, capture, replay
+
+
+FLAGS = [[1, 0], [0, 1], [1, 1], [0, 0], [1, 0], [0, 1], [0, 0]]
+
+
+@pytest.mark.parametrize("warmed_up", [False, True])
+def test_a_captured_launch_uploads_the_descriptors_of_each_replay(monkeypatch, warmed_up):
+    """prepare() and replay() in turn: the graph that captured launch() holds the upload, whether or not a
+    prepare() was pending when it was captured."""
+    opt, capture, replay = _optimizer_on_a_fake_device(monkeypatch)
+    if warmed_up:
+        opt.step(1e-3, [1, 1], [1, 1])
+    else:
+        opt.prepare([1, 1], [1, 1])
+    with capture():
+        opt.launch(1e-3)
+    opt.seen.clear()
+    for f in FLAGS:
+        opt.prepare([1, 1], f)
+        replay()
+    assert opt.seen == FLAGS
+
+
+def test_an_upload_before_the_capture_stays_out_of_the_graph(monkeypatch):
+    """prepare(), upload() and replay() in turn, as StackedMAG does: the rows of the ring are used in turn and
+    the graph copies none of them; eager steps before and after use their own."""
+    opt, capture, replay = _optimizer_on_a_fake_device(monkeypatch)
+    opt.step(1e-3, [1, 1], [1, 1])
+    opt.prepare([1, 1], [0, 0])
+    opt.upload()
+    with capture():
+        opt.launch(1e-3)
+    opt.seen.clear()
+    rows = set()
+    for f in FLAGS:
+        opt.prepare([1, 1], f)
+        opt.upload()
+        rows.add(opt._row)
+        replay()
+    assert opt.seen == FLAGS and len(rows) > 1
+    opt.step(1e-3, [1, 1], [0, 1])
+    opt.launch(1e-3)                       # the same descriptors again
+    assert opt.seen[-2:] == [[0, 1], [0, 1]]
