@@ -49,8 +49,8 @@ def call(name: str, **kw):
     try:
         args = [kw[an] for an, _ in params]
     except KeyError:
-        args = ()
-    if len(args) != len(kw):
+        args = None
+    if args is None or len(args) != len(kw):
         names = [an for an, _ in params]
         raise TypeError(f"{name}: missing {[a for a in names if a not in kw]}, "
                         f"unexpected {[a for a in kw if a not in names]}")
@@ -65,7 +65,13 @@ def call(name: str, **kw):
     bind_stream()
     if ret is None:
         ffi.lib().nlh_clear_status()   # void entries report through the recorded status
-    rc = fn(*args)
+    try:
+        rc = fn(*args)
+    except C.ArgumentError:
+        for at, v in zip(fn.argtypes, args):
+            if at is not C.c_void_p:
+                at(v)                      # a number of the wrong kind is a TypeError
+        raise
     if ret is C.c_int32:
         if rc:
             ffi.check(rc, name)

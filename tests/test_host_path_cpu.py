@@ -251,3 +251,21 @@ def test_an_upload_before_the_capture_stays_out_of_the_graph(monkeypatch):
     opt.step(1e-3, [1, 1], [0, 1])
     opt.launch(1e-3)                       # the same descriptors again
     assert opt.seen[-2:] == [[0, 1], [0, 1]]
+
+
+def test_call_refuses_wrong_arguments_with_a_type_error(monkeypatch):
+    """Names are checked before anything else, an empty call's too; a value that its C type cannot hold
+    raises TypeError, a pointer of an unknown kind ctypes.ArgumentError."""
+    import ctypes
+    from nl_hecate_b200 import dispatch as D
+    bound = []
+    monkeypatch.setattr(D, "bind_stream", lambda: bound.append(1))
+    for kw in ({}, {"option": 3}, {"option": 3, "valu": 1}, {"option": 3, "value": 1, "more": 0}):
+        with pytest.raises(TypeError, match="missing"):
+            D.call("nlh_set_option", **kw)
+    assert not bound
+    with pytest.raises(TypeError):
+        D.call("nlh_set_option", option=3.0, value=1)
+    with pytest.raises(ctypes.ArgumentError):
+        D.call("nlh_simple_rng_fill", state=1.5, scale=1.0, out_host=None, n=0)
+    assert D.call("nlh_set_option", option=torch.tensor(3), value=True) == 0
