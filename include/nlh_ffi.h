@@ -505,7 +505,7 @@ int32_t nlh_cross_entropy_forward(const void* logits, int32_t logits_is_bf16, co
 int32_t nlh_cross_entropy_backward(const void* logits, int32_t logits_is_bf16, const int32_t* target_ids,
     const float* lse, const float* grad_scale, void* d_logits, int32_t n, int32_t vocab, float inv_count);
 
-/* dst [rows, row_len] <- rows of row_len floats, src_stride floats apart. */
+/* dst [rows, row_len] <- rows of row_len floats, src_stride >= row_len floats apart. */
 int32_t nlh_copy_rows(const float* src, int64_t src_stride, float* dst, int32_t rows, int32_t row_len);
 /* dst [cols, rows] <- src [rows, cols] transposed. */
 int32_t nlh_transpose(const float* src, float* dst, int32_t rows, int32_t cols);

@@ -14,6 +14,7 @@
 //                the gradient over the logits in place (bf16 or fp32).
 //   embedding  : 16-byte gathers; scatter-add with vector atomics.
 #include <cuda_bf16.h>
+#include <limits.h>
 #include <math_constants.h>
 
 #include "nlh_common.cuh"
@@ -788,7 +789,7 @@ int32_t nlh_cross_entropy_backward(const void* logits, int32_t logits_is_bf16, c
 
 int32_t nlh_copy_rows(const float* src, int64_t src_stride, float* dst, int32_t rows, int32_t row_len)
 {
-    if (rows < 0 || row_len < 0 || src_stride < 0 || !src || !dst) return NLH_ERR_INVALID_ARG;
+    if (rows < 0 || row_len < 0 || src_stride < row_len || !src || !dst) return NLH_ERR_INVALID_ARG;
     if (rows == 0 || row_len == 0) return NLH_OK;
     if ((((uintptr_t)src | (uintptr_t)dst) & 15) || (src_stride & 3) || (row_len & 3)) {
         const cudaError_t e = cudaMemcpy2DAsync(dst, (size_t)row_len * 4, src, (size_t)src_stride * 4, (size_t)row_len * 4,
@@ -796,7 +797,7 @@ int32_t nlh_copy_rows(const float* src, int64_t src_stride, float* dst, int32_t 
         if (e != cudaSuccess) record_status(NLH_ERR_CUDA, "nlh_copy_rows", cudaGetErrorString(e));
         return e == cudaSuccess ? NLH_OK : NLH_ERR_CUDA;
     }
-    const int row4 = row_len >> 2, per_row = (row4 + 1023) / 1024;
+    const int row4 = row_len >> 2, per_row = min((row4 + 1023) / 1024, max(INT_MAX / rows, 1));   // grid.x < 2^31
     copy_rows_kernel<<<(unsigned)rows * per_row, 256, 0, current_stream()>>>(
         (const float4*)src, src_stride >> 2, (float4*)dst, row4, per_row);
     return check_launch("nlh_copy_rows") ? NLH_OK : NLH_ERR_CUDA;

@@ -252,3 +252,28 @@ def test_model_loss_with_fused_glue_matches_torch_glue():
         res.append((float(loss), m.opt.g.clone()))
     assert abs(res[0][0] - res[1][0]) <= 1e-4 * abs(res[1][0])
     assert rel_err(_np(res[0][1]), _np(res[1][1])) <= 2e-3
+
+
+@pytest.mark.parametrize("rows,row_len,stride,offset", [
+    (3, 1, 1, 0), (3, 1, 5, 0), (2, 3, 7, 1), (5, 4, 4, 0), (5, 4, 12, 0), (4, 8, 8, 1), (3, 6, 8, 0),
+    (3, 4096, 8192, 0), (3, 4100, 4100, 0), (2, 4100, 4104, 2), (1, 12, 12, 0)])
+def test_copy_rows(rows, row_len, stride, offset):
+    """Row lengths around one 16-byte unit and one 1024-unit part, strides above the length, and sources off
+    the 16-byte boundary (the 2D copy): the rows and nothing beside them."""
+    import torch
+    from nl_hecate_b200 import dispatch as D
+    src = torch.arange(offset + rows * stride + 4, device="cuda", dtype=torch.float32)
+    dst = torch.full((rows * row_len + 8,), -1.0, device="cuda")
+    D.call("nlh_copy_rows", src=src.data_ptr() + 4 * offset, src_stride=stride, dst=dst, rows=rows, row_len=row_len)
+    want = src[offset:offset + rows * stride].view(rows, stride)[:, :row_len].reshape(-1)
+    assert torch.equal(dst[:rows * row_len], want) and bool((dst[rows * row_len:] == -1).all())
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (1, 65), (65, 1), (63, 130), (64, 64), (65, 64), (512, 8192)])
+def test_transpose(rows, cols):
+    import torch
+    from nl_hecate_b200 import dispatch as D
+    src = torch.randn(rows, cols, device="cuda")
+    dst = torch.full((rows * cols + 8,), -1.0, device="cuda")
+    D.call("nlh_transpose", src=src, dst=dst, rows=rows, cols=cols)
+    assert torch.equal(dst[:rows * cols].view(cols, rows), src.t()) and bool((dst[rows * cols:] == -1).all())

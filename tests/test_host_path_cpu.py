@@ -269,3 +269,10 @@ def test_call_refuses_wrong_arguments_with_a_type_error(monkeypatch):
     with pytest.raises(ctypes.ArgumentError):
         D.call("nlh_simple_rng_fill", state=1.5, scale=1.0, out_host=None, n=0)
     assert D.call("nlh_set_option", option=torch.tensor(3), value=True) == 0
+
+
+def test_copy_rows_refuses_overlapping_rows():
+    """Rows closer than their length are refused whatever their alignment, before anything is launched."""
+    from nl_hecate_b200 import ffi
+    for stride, row_len in ((4, 8), (0, 4), (2, 3), (-4, 4)):
+        assert ffi.lib().nlh_copy_rows(64, stride, 64, 2, row_len) == ffi.lib().nlh_copy_rows(64, 4, 64, -1, 4)
