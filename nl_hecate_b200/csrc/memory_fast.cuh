@@ -752,8 +752,8 @@ __global__ void __launch_bounds__(FastGeom<D, SPLIT>::NT, (D == 64 && !FROZEN) ?
         __syncthreads();
     }
 
+    if (a.d_m_out == nullptr) return;   // initial-state gradients not requested
     if (a.atomic_out) {
-        if (a.d_m_out == nullptr) return;   // batch-summed initial-state gradients not requested
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             // physical pair i holds logical elements 2i ^ (xc << 2) and the next one

@@ -314,6 +314,27 @@ def test_recompute_training_pair_exact(D, orc, rule, d, s, interval, n):
         assert rel_err(_np(g[key]), w[key]) <= REL, key
 
 
+@pytest.mark.parametrize("rule,chunk", [(0, 0), (1, 0), (2, 0), (0, 8), (1, 8), (1, 16)])
+@pytest.mark.parametrize("d", [16, 32, 64, 128])
+def test_per_problem_backward_without_initial_gradients(D, orc, rule, chunk, d):
+    """nlh_rule_backward with d_m_initial = d_s_initial = NULL: they are not computed, the rest is the same."""
+    import torch
+    n, s, interval = 2, 19, chunk or 8
+    t = to_dev(make_problem(orc, n, s, d, 1800 + d, "rand"))
+    mc, sc, _ = D.rule_forward(rule, t["k"], t["v"], t["q"], t["alpha"], t["theta"], t["eta"], t["m0"], t["s0"],
+                               interval, chunk)
+    ref = D.rule_backward(rule, t["k"], t["v"], t["q"], t["alpha"], t["theta"], t["eta"], mc, sc, t["dy"], interval, chunk)
+    dk, dv, dq = (torch.empty_like(t["k"]) for _ in range(3))
+    da, dt, de = (torch.empty_like(t["alpha"]) for _ in range(3))
+    D.call("nlh_rule_backward", rule=rule, k_mem=t["k"], v_mem=t["v"], q_mem=t["q"], alpha=t["alpha"],
+           theta=t["theta"], eta=t["eta"], m_ckpt=mc, s_ckpt=sc, d_y=t["dy"], d_k_mem=dk, d_v_mem=dv, d_q_mem=dq,
+           d_alpha=da, d_theta=dt, d_eta=de, d_m_initial=None, d_s_initial=None, seq_len=s, d=d, batch_size=n,
+           interval=interval, chunk_size=chunk, error_clip=0.0, m_norm_max=0.0)
+    for key, got in dict(d_k=dk, d_v=dv, d_q=dq, d_alpha=da, d_theta=dt, d_eta=de).items():
+        if ref[key] is not None:
+            assert rel_err(_np(got), _np(ref[key])) <= 1e-6, key
+
+
 @pytest.mark.parametrize("d,s,chunk,n", [(64, 48, 16, 2), (64, 20, 8, 3)])
 def test_recompute_training_pair_frozen(D, orc, d, s, chunk, n):
     p = make_problem(orc, n, s, d, 1900 + d + s, "rand")
