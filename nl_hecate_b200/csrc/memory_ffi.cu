@@ -156,7 +156,7 @@ static BwdArgs bwd_args(const float* k, const float* v, const float* q, const fl
     a.m_traj = m_traj; a.s_traj = s_traj; a.d_y = d_y; a.d_m_seed = d_m_seed; a.d_s_seed = d_s_seed;
     a.d_k = d_k; a.d_v = d_v; a.d_q = d_q; a.d_alpha = d_alpha; a.d_theta = d_theta; a.d_eta = d_eta;
     a.d_m_out = d_m_out; a.d_s_out = d_s_out;
-    a.dM = a.dS = a.dM0 = a.m_rec = a.s_rec = nullptr;
+    a.dM = a.dS = a.dM0 = a.m_rec = a.s_rec = a.part = nullptr;
     a.seq_len = seq_len; a.d = d; a.batch = batch; a.t_start = t_start; a.t_end = t_end;
     a.traj_stride = traj_stride; a.frozen = frozen; a.chunk = chunk; a.atomic_out = atomic_out;
     a.error_clip = clip; a.m_norm_max = mmax;

@@ -82,6 +82,7 @@ struct BwdArgs {
     int frozen, chunk;
     int atomic_out;                // 1: atomicAdd into one shared [d*d]; 0: store per batch element
     float error_clip, m_norm_max;
+    float* part;                   // work: sums of the CTAs of a problem whose rows are divided (d = 128)
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
