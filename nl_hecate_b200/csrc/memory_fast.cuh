@@ -859,10 +859,13 @@ inline int sm_count()
 // problems two CTAs would share an SM and nothing is gained).
 inline bool split_rows(int d, int batch) { return d == 64 && 2 * batch <= sm_count() && option_value(NLH_OPT_ROW_SPLIT) != 0; }
 
-// Rows of a D = 128 problem per CTA: 16 while all CTAs then still find room at once (two per SM), else
-// 32. The kernels are bound by the token chain of a CTA when few CTAs run, by the k/v/q streams that
-// every CTA of a problem reads again when many do.
-inline bool split_128_fine(int batch) { return batch * 8 <= 2 * sm_count(); }
+// CTAs per D = 128 problem: 8 (16 rows each) while every CTA gets an SM of its own, else 4. A CTA's token
+// chain is the shorter the fewer rows it has; but the CTAs of a problem read the same k/v/q streams again, and from
+// the second CTA on an SM (or, Titans backward, the second wave: 117 KB of shared memory) the wider split loses.
+// us with 8 / 4 CTAs on 148 SMs: Delta backward, 512 tokens, 18 problems 415 / 469, 20 544 / 492, 37 551 / 493;
+// Titans backward, 256 tokens, 18 problems 254 / 319, 20 438 / 320, 37 436 / 312; forward Delta 183 / 227, 232 / 230,
+// 234 / 230; forward Titans 121 / 185, 186 / 187, 234 / 231.
+inline bool split_128_fine(int batch) { return batch * 8 <= sm_count(); }
 
 template <int RULE, bool FROZEN, int SPLIT>
 static void fwd128_launch(const FwdArgs& a, cudaStream_t st)
