@@ -867,24 +867,29 @@ inline bool split_rows(int d, int batch) { return d == 64 && 2 * batch <= sm_cou
 // 234 / 230; forward Titans 121 / 185, 186 / 187, 234 / 231.
 inline bool split_128_fine(int batch) { return batch * 8 <= sm_count(); }
 
-template <int RULE, bool FROZEN, int SPLIT>
+template <int RULE, bool FROZEN, int SPLIT, bool BULK>
 static void fwd128_launch(const FwdArgs& a, cudaStream_t st)
 {
     const size_t smem = fast_fwd_smem_floats<128>() * sizeof(float);
-    cudaFuncSetAttribute(fast_fwd_kernel<128, RULE, FROZEN, SPLIT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fast_fwd_kernel<128, RULE, FROZEN, SPLIT, true><<<a.batch * SPLIT, FastGeom<128, SPLIT>::NT, smem, st>>>(a);
+    cudaFuncSetAttribute(fast_fwd_kernel<128, RULE, FROZEN, SPLIT, BULK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    fast_fwd_kernel<128, RULE, FROZEN, SPLIT, BULK><<<a.batch * SPLIT, FastGeom<128, SPLIT>::NT, smem, st>>>(a);
 }
-template <int RULE>
+template <int RULE, bool BULK>
 static bool fast_fwd_launch_128(const FwdArgs& a, cudaStream_t st)
 {
     if constexpr (RULE != RULE_HEBBIAN) {
         if (a.frozen) {
-            if (split_128_fine(a.batch)) fwd128_launch<RULE, true, 8>(a, st); else fwd128_launch<RULE, true, 4>(a, st);
+            if (split_128_fine(a.batch)) fwd128_launch<RULE, true, 8, BULK>(a, st); else fwd128_launch<RULE, true, 4, BULK>(a, st);
             return true;
         }
     }
-    if (split_128_fine(a.batch)) fwd128_launch<RULE, false, 8>(a, st); else fwd128_launch<RULE, false, 4>(a, st);
+    if (split_128_fine(a.batch)) fwd128_launch<RULE, false, 8, BULK>(a, st); else fwd128_launch<RULE, false, 4, BULK>(a, st);
     return true;
+}
+template <int RULE>
+static bool fast_fwd_launch_128(const FwdArgs& a, cudaStream_t st)
+{
+    return option_value(NLH_OPT_BULK_STAGING) ? fast_fwd_launch_128<RULE, true>(a, st) : fast_fwd_launch_128<RULE, false>(a, st);
 }
 
 template <int D, int RULE>

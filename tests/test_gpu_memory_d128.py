@@ -130,6 +130,24 @@ def test_segment_backward_leaves_the_other_tokens_alone(D, orc, rule, t0, t1):
             assert rel_err(got[:, t0:t1], ref[key.replace("_mem", "")]) <= REL, key
 
 
+@pytest.mark.parametrize("n,s", [(2, 5), (3, 37), (19, 16), (40, 33)])
+def test_both_stagings_of_the_forward_give_the_same_bits(D, orc, n, s):
+    """NLH_OPT_BULK_STAGING = 0: cp.async in place of bulk copies, exact and frozen, both splits."""
+    t = to_dev(make_problem(orc, n, s, DIM, 6600 + n + s, "rand"))
+    out = []
+    for on in (1, 0):
+        D.call("nlh_set_option", option=5, value=on)
+        try:
+            out.append([x for rule, chunk in ((0, 0), (1, 0), (2, 0), (0, 8), (1, 8)) for x in
+                        D.rule_forward(rule, *(t[k] for k in ("k", "v", "q", "alpha", "theta", "eta", "m0", "s0")), 8, chunk)
+                        if x is not None])
+        finally:
+            D.call("nlh_set_option", option=5, value=1)
+    for x, y in zip(*out):
+        assert np.array_equal(_np(x), _np(y))
+    assert D.call("nlh_bulk_timeout_flag") == 0
+
+
 def test_clipped_rule_at_the_same_size_runs_the_generic_kernels(D, orc):
     p = make_problem(orc, 2, 12, DIM, 6700, "const", scale=1.0, state_scale=1.0)
     w = oracle_exact(orc, "titans", p, error_clip=1.0, m_norm_max=5.0)
