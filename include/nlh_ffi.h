@@ -314,7 +314,9 @@ int32_t nlh_swa_backward_f32(const float* q, const float* k, const float* v, con
  * waits ran out (0 = never, 1 = a wait expired and results are invalid, -1 = read failed). */
 #define NLH_OPT_SWA_TCGEN05 1
 /* NLH_OPT_CHUNK_MATRIX (default 1): frozen-M0 chunkwise Titans / Delta entries at head_dim 64 and
- * chunk sizes 16..64 run in matrix form on the tensor cores; 0 selects the per-token kernels. */
+ * chunk sizes 16..64 run in matrix form on the tensor cores; 0 selects the per-token kernels. Operands there
+ * are split fp32: below 2^-110 they lose low bits, finite ones above 3.39e38 become NaN. A NaN or an infinity
+ * reaches the outputs that it reaches token by token, and no others; an infinity may arrive as a NaN. */
 #define NLH_OPT_CHUNK_MATRIX 2
 /* NLH_OPT_ROW_SPLIT (default 1): when a launch has at most half as many problems as the GPU has SMs, the exact
  * head_dim-64 forward and the M-only exact Titans backward divide every problem's rows over two

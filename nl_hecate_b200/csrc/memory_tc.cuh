@@ -26,15 +26,18 @@
 // hi.hi, hi.mid, mid.hi, mid.mid, hi.lo, lo.hi accumulated in fp32 in TMEM, the small ones first (the
 // dropped ones are below 2^-24 of the product). Scans and gate tables are fp32 FMA. Against float64, 16
 // problems x 333 tokens, chunk 64: y 1.25e-7, dK 2.0e-7, dV 1.8e-7, d_eta 2.0e-7 (fp32 FMA contractions, which
-// these replace: 1.6e-7, 3.1e-7, 2.1e-7, 2.4e-7). The exact rule has the same form with a triangular solve per
+// these replace: 1.6e-7, 3.1e-7, 2.1e-7, 2.4e-7). All 24 bits are there while the low plane is a normal bf16: an
+// operand below 2^-110 keeps fewer. One that rounds above the largest bf16 (3.39e38), and an infinity, become NaN.
+// Values that are not finite reach the tokens that the per-token statement lets them reach and no others
+// (NonFinite below). The exact rule has the same form with a triangular solve per
 // tile, but there it replaces per-token kernels at 1.0e-7 and came to 2.1e-7: it stays with those.
 //
 // What bounds it. One CTA (256 threads) walks one problem, so a launch is bound by the chain of a
-// tile's stages: tensor products (55 cycles per 128x64x16 plane product, the A operand is read from
-// shared memory for each; 22k of a backward tile's cycles), loads and the conversion of every intermediate
+// tile's stages: tensor products (55 cycles per 128x64x16 plane product, 64 per 128x128x16, the A operand is
+// read from shared memory for each; the 312 of a Titans backward tile take 17.6k of its 51k cycles), loads and the conversion of every intermediate
 // into planes with two warps per scheduler. The stage times are the same with 4 problems as with 128, so
 // neither memory nor the other SMs bound them. Forward and backward, 128 problems x 2048 tokens, chunk 64:
-// 1802 us with fp32 FMA contractions in shared memory, 1177 us so (Delta, 24 x 1000, chunk 48: 903 -> 633).
+// 1802 us with fp32 FMA contractions in shared memory, 1184 us so (Delta, 24 x 1000, chunk 48: 903 -> 633).
 //
 // Shared-memory matrices: element (row, col) of an R-row plane at (col/8)*(R*16) + row*16 + (col%8)*2,
 // the canonical no-swizzle core-matrix layout with the 8-column chunk outermost. The same bytes serve
@@ -146,7 +149,7 @@ struct Tables {
     unsigned tmem;
 };
 
-// W of the tile as a table [TMAX][LDX], row t: W(t, j), zero above the diagonal; tb.ab[t] = A_t, B_t;
+// W of the tile as a table [TMAX][LDX], row t: W(t, j), of no meaning above the diagonal; tb.ab[t] = A_t, B_t;
 // tb.wS[j] = theta_j h(j, L-1); tb.tot = A_L, B_L, H_L; tb.wM = W(L-1, .). One thread per column j, the
 // recurrence runs over t: h' = eta_t h, Om' = r_t Om + h'. With one row per thread (63 unrolled steps in
 // every warp) this stage took the MMA-issuing warp, which the others wait for, 4.6k cycles a tile; 2.8k so.
@@ -161,17 +164,16 @@ __device__ __forceinline__ void decay_table(Tables& tb, float* Wt, int tid, int 
         for (int t = 0; t < TMAX; t++) {
             const float4 g = tb.gt[t];
             h = t == j ? 1.f : g.y * h;
-            om = fmaf(g.x, om, h);
-            if (!HAS_S) om = t == j ? 1.f : om;
+            om = t == j ? 1.f : fmaf(g.x, om, h);      // starts here, whatever the gates before j hold
             Wt[t * LDX + j] = th * om;
-            if (t == L - 1) { tb.wM[j] = th * om; if (HAS_S) tb.wS[j] = th * h; }
+            if (t == L - 1) { tb.wM[j] = t >= j ? th * om : 0.f; if (HAS_S) tb.wS[j] = t >= j ? th * h : 0.f; }
         }
     } else if (tid == TMAX) {
         float aa = 1.f, h = 1.f, om = 0.f;
 #pragma unroll 8
         for (int t = 0; t < TMAX; t++) {
             const float4 g = tb.gt[t];
-            aa *= g.x; h *= g.y; om = fmaf(g.x, om, h);
+            aa *= g.x; h *= g.y; om = t == 0 ? h : fmaf(g.x, om, h);
             tb.ab[t] = make_float2(aa, HAS_S ? om : 0.f);
             if (t == L - 1) { tb.tot[0] = aa; tb.tot[1] = HAS_S ? om : 0.f; tb.tot[2] = h; }
         }
@@ -264,6 +266,44 @@ struct Waiter {
         fence_after_sync();
     }
 };
+// ── values that are not finite ──
+// W is zero above the diagonal, but 0 x NaN in a 64-token product would carry a token's NaN or infinity to
+// the tokens on the wrong side of it. Elementwise products with W select; a product over tokens whose
+// other operand holds such a value is formed again over the tokens that belong to it, in fp32 FMA.
+struct NonFinite {
+    float z = 0.f;
+    __device__ __forceinline__ void add(const float (&v)[8])
+    {
+#pragma unroll
+        for (int j = 0; j < 8; j++) z = fmaf(v[j], 0.f, z);
+    }
+    __device__ __forceinline__ bool any() const { return !(z == 0.f); }
+};
+__device__ __forceinline__ float plane_element(const unsigned char* t, int R, int plane, int row, int col)
+{
+    const unsigned char* p = t + (col >> 3) * (R * 16) + row * 16 + (col & 7) * 2;
+    auto f = [](const unsigned char* q) { return __uint_as_float((unsigned)*reinterpret_cast<const unsigned short*>(q) << 16); };
+    return (f(p + 2 * plane) + f(p + plane)) + f(p);
+}
+// s = sum over tokens j0 <= j < j1 of a(j) times 32 columns of token j; b(v, j, c): 8 columns from chunk c of 4
+template <class A, class B>
+__device__ __forceinline__ void sum_tokens(float (&s)[32], int j0, int j1, A a, B b)
+{
+#pragma unroll
+    for (int i = 0; i < 32; i++) s[i] = 0.f;
+#pragma unroll 1
+    for (int j = j0; j < j1; j++) {
+        const float w = a(j);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            float v[8];
+            b(v, j, c);
+#pragma unroll
+            for (int i = 0; i < 8; i++) s[8 * c + i] = fmaf(w, v[i], s[8 * c + i]);
+        }
+    }
+}
+
 // all generic-proxy writes to shared memory and TMEM reads so far are ordered before the MMAs that one
 // thread issues after it
 __device__ __forceinline__ void publish()
@@ -271,6 +311,13 @@ __device__ __forceinline__ void publish()
     fence_async_proxy();
     fence_before_sync();
     __syncthreads();
+}
+// the same, and whether any thread found something
+__device__ __forceinline__ bool publish_or(bool found)
+{
+    fence_async_proxy();
+    fence_before_sync();
+    return __syncthreads_or(found) != 0;
 }
 
 // ───────────────────────────────── forward ─────────────────────────────────
@@ -366,7 +413,7 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
         tload(acc, trow);
 #pragma unroll
         for (int i = 0; i < 32; i++) acc[i] *= au;
-        if (HAS_S) {
+        if (HAS_S && !krow) {
             tload(p, trow + 64);
 #pragma unroll
             for (int i = 0; i < 32; i++) acc[i] = fmaf(bu, p[i], acc[i]);
@@ -381,18 +428,20 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
             st32(Xb + tr * LDX + hf * 32, acc);
         } else {
 #pragma unroll
-            for (int i = 0; i < 32; i++) p[i] *= -w[i];
+            for (int i = 0; i < 32; i++) p[i] = hf * 32 + i <= tr ? p[i] * -w[i] : 0.f;
             store32(sm + F_WP, 64, 8192, tr, hf * 4, p);
         }
         if (c + 1 < ntile) fetch(c + 1);         // lands under the products
         __syncthreads();
         // E and its tile-end weighted copies as planes
+        NonFinite nf;
 #pragma unroll 1
         for (int i = 0; i < 2; i++) {
             const int row = un.row(i);
             const float wm = tb.wM[row], wsv = HAS_S ? tb.wS[row] : 0.f;
             float e[8], s[8];
             ld8(e, Xb + row * LDX + un.cc * 8);
+            nf.add(e);
             store8(sm + F_E, 64, 8192, row, un.cc, e);
 #pragma unroll
             for (int j = 0; j < 8; j++) s[j] = e[j] * wm;
@@ -403,7 +452,7 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
                 store8(sm + F_EW, 64, 16384, row, 8 + un.cc, s);
             }
         }
-        publish();
+        const bool again = publish_or(nf.any());
         if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<true, true>(tm + 256, ew, 16384, 64, kq, 16384, 128, 64);              // [Ew Es]^T K
@@ -437,6 +486,9 @@ __global__ void __launch_bounds__(NT, 1) tile_fwd_kernel(FwdArgs a, int T)
         wait(2);
         tload(p, trow + 192);
         if (!krow) {
+            if (again)
+                sum_tokens(p, 0, tr + 1, [&](int j) { return plane_element(sm + F_WP, 64, 8192, tr, j); },
+                           [&](float (&v8)[8], int j, int c8) { ld8(v8, Xb + j * LDX + hf * 32 + c8 * 8); });
 #pragma unroll
             for (int i = 0; i < 32; i++) p[i] += acc[i];
             st32(Yb + tr * LDX + hf * 32, p);          // and so have the errors
@@ -532,6 +584,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
         // ── stage 1: operands; K K^T | Q K^T and K,Q x M0,S0 ──
         // The four units of each matrix go round one loop with the next unit's loads in flight (as fast as
         // straight-line code with all 24 loads at once, 8k cycles a tile, and a third of its size).
+        NonFinite nf;                                // in K, Q, dY
         {
             float x[8], y[8], x3[8];
             auto get = [&](int i) {                  // K, V, M0 rows, then Q, dY, S0 rows
@@ -551,6 +604,8 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
                     xc[j] = in ? x[j] : 0.f; yc[j] = in ? y[j] : 0.f; x3c[j] = x3[j];
                 }
                 if (i < 3) get(i + 1);
+                nf.add(xc);
+                if (i >= 2) nf.add(yc);
                 store8(kqp, 128, 16384, r, un.cc, xc);
                 store8(xxp, 128, 16384, r, un.cc, x3c);
                 if (i < 2) st8(Xb + r * LDX + un.cc * 8, yc);
@@ -561,7 +616,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             tb.gt[tid] = make_float4(1.0f - gal, get, gth, 0.f);
             if (c > 0) fetch_gates(c - 1);
         }
-        publish();
+        const bool again = publish_or(nf.any());
         if (warp == 0 && elect_one()) {
             fence_after_sync();
             mma6<false, false>(tm, kq, 16384, 128, kq, 16384, 128, 64);
@@ -606,14 +661,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const float4 v4 = *reinterpret_cast<const float4*>(Xb + tr * LDX + hf * 32 + 4 * i);
-                    acc[4 * i] = fmaf(au, acc[4 * i], -v4.x); acc[4 * i + 1] = fmaf(au, acc[4 * i + 1], -v4.y);
-                    acc[4 * i + 2] = fmaf(au, acc[4 * i + 2], -v4.z); acc[4 * i + 3] = fmaf(au, acc[4 * i + 3], -v4.w);
-                }
-                if (HAS_S) {
-                    float s[32];
-                    tload(s, trow + 128);
-#pragma unroll
-                    for (int i = 0; i < 32; i++) acc[i] = fmaf(bu, s[i], acc[i]);
+                    acc[4 * i] -= v4.x; acc[4 * i + 1] -= v4.y; acc[4 * i + 2] -= v4.z; acc[4 * i + 3] -= v4.w;
                 }
                 st32(Xb + tr * LDX + hf * 32, acc);
             } else {
@@ -641,7 +689,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
         if (!krow) {
             float wpv[32];
 #pragma unroll
-            for (int i = 0; i < 32; i++) wpv[i] = w[i] * p[i];
+            for (int i = 0; i < 32; i++) wpv[i] = hf * 32 + i <= tr ? w[i] * p[i] : 0.f;
             store32(sm + B_WZ + 24576, 64, 8192, tr, hf * 4, wpv);
         }
         store32(xxp, 128, 16384, R, hf * 4, g);
@@ -662,6 +710,9 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             float s[32];
             tload(dx, trow);
             tload(s, trow + 128);
+            if (again)
+                sum_tokens(s, tr, L, [&](int t) { return plane_element(sm + B_WZ + 24576, 64, 8192, t, tr); },
+                           [&](float (&v8)[8], int t, int c8) { load8(v8, yfp, 128, 16384, 64 + t, hf * 4 + c8); });
 #pragma unroll
             for (int i = 0; i < 32; i++) dx[i] = -fmaf(wm, dx[i], s[i]);
             if (HAS_S) {
@@ -734,7 +785,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             float s[32];
             tload(s, trow);                            // N row (krow) or R row
 #pragma unroll
-            for (int i = 0; i < 32; i++) { p[i] *= s[i]; s[i] *= -w[i]; }
+            for (int i = 0; i < 32; i++) { p[i] *= s[i]; s[i] = hf * 32 + i <= tr ? s[i] * -w[i] : 0.f; }
             if (!krow) store32(sm + B_WZ, 128, 16384, R, hf * 4, s);
             wait(1);
             if (!krow) {
@@ -746,11 +797,13 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             }
             float s2[32];
             tload(s, trow + 64);
-            if (HAS_S) tload(s2, trow + 128);
+            if (krow) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-                dx[i] = krow ? fmaf(au, s[i], dx[i]) : au * s[i];
-                if (HAS_S) dx[i] = fmaf(bu, s2[i], dx[i]);
+                for (int i = 0; i < 32; i++) dx[i] += s[i];
+            } else {
+                if (HAS_S) tload(s2, trow + 128);
+#pragma unroll
+                for (int i = 0; i < 32; i++) dx[i] = HAS_S ? fmaf(bu, s2[i], au * s[i]) : au * s[i];
             }
         }
         publish();
@@ -805,7 +858,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             const float* xs = Ss + (tr + 1) * LDS + hf * 32;
             if (tr + 1 < L) {
 #pragma unroll
-                for (int i = 0; i < 32; i++) s1 = fmaf(w[i], xd[i], s1);     // w is zero above the diagonal
+                for (int i = 0; i < 32; i++) s1 = hf * 32 + i <= tr ? fmaf(w[i], xd[i], s1) : s1;
                 if (HAS_S) {
                     float hh = 1.f;
                     const int jh = hf * 32;
@@ -842,6 +895,10 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
         {
             float s[32];
             tload(s, trow + (krow ? 256 : 192));
+            if (again)                                 // dK: tokens from this one on; dQ: tokens up to this one
+                sum_tokens(s, krow ? tr : 0, krow ? L : tr + 1,
+                           [&](int j) { return plane_element(sm + B_WZ, 128, 16384, 64 + (krow ? j : tr), krow ? tr : j); },
+                           [&](float (&v8)[8], int j, int c8) { load8(v8, kqp, 128, 16384, (krow ? 64 : 0) + j, hf * 4 + c8); });
 #pragma unroll
             for (int i = 0; i < 32; i++) dx[i] += s[i];
         }
@@ -856,7 +913,7 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
             store8(sm + B_WZ, 128, 32768, R, hf * 4 + c8, s);
             if (HAS_S) {
 #pragma unroll
-                for (int i = 0; i < 8; i++) s[i] = f[i] * bu;
+                for (int i = 0; i < 8; i++) s[i] = krow ? 0.f : f[i] * bu;
                 store8(sm + B_WZ, 128, 32768, R, 8 + hf * 4 + c8, s);
             }
         }
@@ -879,6 +936,12 @@ __global__ void __launch_bounds__(NT, 1) tile_bwd_kernel(BwdArgs a, int T)
         {
             float s[32];
             tload(s, trow + 320);
+            if (again && HAS_S) {
+                if (!krow)                             // without the K rows, whose weights for G_S are zero
+                    sum_tokens(s, 0, L, [&](int t) { return plane_element(sm + B_WZ, 128, 32768, 64 + t, 64 + tr); },
+                               [&](float (&v8)[8], int t, int c8) { load8(v8, kqp, 128, 16384, 64 + t, hf * 4 + c8); });
+                __syncthreads();                       // the staged rows below go over those weights
+            }
             if (HAS_S || krow) {
 #pragma unroll
                 for (int i = 0; i < 32; i++) g[i] += s[i];

@@ -177,6 +177,44 @@ def test_chunk_tiles_at_their_edges(D, orc, rule, s, chunk):
     _check_bwd(g, w, ["d_k", "d_v", "d_q", "d_alpha", "d_theta"] + (["d_eta"] if r else []), tol_abs=1e-3)
 
 
+@pytest.mark.parametrize("rule", ["titans", "delta"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("where", ["k", "v", "q", "dy", "k row", "v row", "q row", "dy row", "alpha", "theta", "eta", "m0", "s0"])
+@pytest.mark.parametrize("s,chunk,token", [(100, 64, 37), (100, 64, 64), (40, 16, 31), (30, 48, 0), (150, 50, 99)])
+def test_chunk_tiles_keep_non_finite_tokens_where_they_belong(D, orc, rule, value, where, s, chunk, token):
+    """One NaN or infinity in one token: the matrix form computes every value that the per-token kernels
+    compute, that is, outputs of the tokens before it (and gradients of the tokens after it) stay finite and
+    right; where those give no finite value, it gives none either."""
+    if rule == "delta" and where in ("eta", "s0"):
+        return
+    p = make_problem(orc, 2, s, 64, 5400 + s + chunk, "rand")
+    name = where.split()[0]
+    if name in ("m0", "s0"):
+        p[name][1, 5 * 64 + 7] = value
+    elif p[name].ndim == 2:
+        p[name][1, token] = value
+    else:
+        p[name][1, token, slice(None) if "row" in where else 11] = value
+    t = to_dev(p)
+    r = 1 if rule == "titans" else 0
+    eta, s0 = (t["eta"], t["s0"]) if r else (None, None)
+    out = []
+    for on in (0, 1):
+        D.call("nlh_set_option", option=2, value=on)
+        try:
+            mc, sc, y = D.rule_forward(r, t["k"], t["v"], t["q"], t["alpha"], t["theta"], eta, t["m0"], s0, chunk, chunk)
+            g = D.rule_backward(r, t["k"], t["v"], t["q"], t["alpha"], t["theta"], eta, mc, sc, t["dy"], chunk, chunk)
+        finally:
+            D.call("nlh_set_option", option=2, value=1)
+        out.append({n: _np(x) for n, x in dict(g, y=y, mc=mc, sc=sc).items() if x is not None})
+    for key, want in out[0].items():
+        got, fin = out[1][key], np.isfinite(want)
+        assert np.isfinite(got[fin]).all(), (key, int((~np.isfinite(got[fin])).sum()), int(fin.sum()))
+        assert not np.isfinite(got[~fin]).any(), (key, int(np.isfinite(got[~fin]).sum()), int((~fin).sum()))
+        if fin.any():
+            assert rel_err(got[fin], want[fin]) <= REL, key
+
+
 def test_chunk1_matches_per_token_kernel(D, orc):
     # core/src/gpu_forward.rs:4193-4300: C=1 chunkwise == per-token kernel (<1e-5)
     p = make_problem(orc, 2, 16, 64, 1200, "const")
