@@ -321,7 +321,9 @@ int32_t nlh_swa_backward_f32(const float* q, const float* k, const float* v, con
 /* NLH_OPT_ROW_SPLIT (default 1): when a launch has at most half as many problems as the GPU has SMs, the exact
  * head_dim-64 forward and the M-only exact Titans backward divide every problem's rows over two
  * CTAs (the rows of the memory evolve independently; the backward then zeroes d_q, d_k and the gate
- * gradients itself and adds the two partial sums into them). 0 keeps one CTA per problem. */
+ * gradients itself and adds the two partial sums into them). 0 keeps one CTA per problem. At head_dim 128 the rows
+ * are divided over 8 or 4 CTAs whatever the option says; the sums are added up in one order there,
+ * in library scratch of 7 or 3 times the gradients d_q, d_k and the gates' own size. */
 #define NLH_OPT_ROW_SPLIT 3
 /* NLH_OPT_SWA_TMA (default 1): the tcgen05 SWA forward stages its Q, K and V tiles with tiled TMA
  * copies (cp.async.bulk.tensor, one issuing thread, completion on an mbarrier; plain single-CTA
@@ -331,7 +333,8 @@ int32_t nlh_swa_backward_f32(const float* q, const float* k, const float* v, con
  * 32/64/128) stage their k, v, q tiles with one bulk asynchronous copy per stream and tile
  * (cp.async.bulk from one thread, completion counted on an mbarrier) instead of per-thread
  * cp.async; 0 selects the cp.async staging. Results are identical. nlh_bulk_timeout_flag() is
- * nonzero if a bounded mbarrier wait of these kernels ever ran out. */
+ * nonzero if a bounded mbarrier wait of these kernels, or of the matrix-form ones
+ * (NLH_OPT_CHUNK_MATRIX), ever ran out. */
 #define NLH_OPT_BULK_STAGING 5
 int32_t nlh_bulk_timeout_flag(void);
 int32_t nlh_set_option(int32_t option, int32_t value);

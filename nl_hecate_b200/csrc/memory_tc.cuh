@@ -34,7 +34,7 @@
 //
 // What bounds it. One CTA (256 threads) walks one problem, so a launch is bound by the chain of a
 // tile's stages: tensor products (55 cycles per 128x64x16 plane product, 64 per 128x128x16, the A operand is
-// read from shared memory for each; the 312 of a Titans backward tile take 17.6k of its 51k cycles), loads and the conversion of every intermediate
+// read from shared memory for each; the 312 of a Titans backward tile take 17.6k of its 47k cycles), loads and the conversion of every intermediate
 // into planes with two warps per scheduler. The stage times are the same with 4 problems as with 128, so
 // neither memory nor the other SMs bound them. Forward and backward, 128 problems x 2048 tokens, chunk 64:
 // 1802 us with fp32 FMA contractions in shared memory, 1184 us so (Delta, 24 x 1000, chunk 48: 903 -> 633).

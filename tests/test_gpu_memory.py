@@ -3,8 +3,8 @@
 Tolerances: forward max-abs 1e-5 and backward max-abs 1e-4 on +-0.1 inputs are
 the reference's own (core/tests/test_cuda_titans.rs:1-4,94-96); relative error
 <= 1e-4 (max-abs error over max-abs reference) is the fp32 bar of the hot path.
-Head dims 32 and 64 without clip/projection run the register-resident kernels,
-everything else the generic-d kernels; both are covered.
+Head dims 32, 64 and 128 without clip/projection run the register-resident kernels (more of 128 in
+test_gpu_memory_d128.py), everything else the generic-d kernels; both are covered.
 """
 import numpy as np
 import pytest
