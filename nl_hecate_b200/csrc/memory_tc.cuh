@@ -34,10 +34,11 @@
 //
 // What bounds it. One CTA (256 threads) walks one problem, so a launch is bound by the chain of a
 // tile's stages: tensor products (55 cycles per 128x64x16 plane product, 64 per 128x128x16, the A operand is
-// read from shared memory for each; the 312 of a Titans backward tile take 17.6k of its 47k cycles), loads and the conversion of every intermediate
-// into planes with two warps per scheduler. The stage times are the same with 4 problems as with 128, so
-// neither memory nor the other SMs bound them. Forward and backward, 128 problems x 2048 tokens, chunk 64:
-// 1802 us with fp32 FMA contractions in shared memory, 1184 us so (Delta, 24 x 1000, chunk 48: 903 -> 633).
+// read from shared memory for each; the 312 of a Titans backward tile take 17.6k of its 47k cycles), loads
+// and the conversion of every intermediate into planes with two warps per scheduler. The stage times are the
+// same with 4 problems as with 128, so neither memory nor the other SMs bound them. Forward and backward,
+// 128 problems x 2048 tokens, chunk 64: 1802 us with fp32 FMA contractions in shared memory, 1172 us so (Delta,
+// 24 x 1000, chunk 48: 903 -> 633).
 //
 // Shared-memory matrices: element (row, col) of an R-row plane at (col/8)*(R*16) + row*16 + (col%8)*2,
 // the canonical no-swizzle core-matrix layout with the 8-column chunk outermost. The same bytes serve
@@ -182,15 +183,20 @@ __device__ __forceinline__ void decay_table(Tables& tb, float* Wt, int tid, int 
 // Row u of the table for this thread's 32 columns (half hf), and A_u, B_u; u = -1: no token before
 __device__ __forceinline__ void decay_row(const Tables& tb, const float* Wt, int u, int hf, float (&w)[32], float& au, float& bu)
 {
-    const float* row = Wt + max(u, 0) * LDX + hf * 32;
-    const float2 ab = tb.ab[max(u, 0)];
+    if (u < 0) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) w[i] = 0.f;
+        au = 1.f; bu = 0.f;
+        return;
+    }
+    const float* row = Wt + u * LDX + hf * 32;
+    const float2 ab = tb.ab[u];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const float4 x = *reinterpret_cast<const float4*>(row + 4 * i);
-        w[4 * i] = u < 0 ? 0.f : x.x; w[4 * i + 1] = u < 0 ? 0.f : x.y; w[4 * i + 2] = u < 0 ? 0.f : x.z; w[4 * i + 3] = u < 0 ? 0.f : x.w;
+        w[4 * i] = x.x; w[4 * i + 1] = x.y; w[4 * i + 2] = x.z; w[4 * i + 3] = x.w;
     }
-    au = u < 0 ? 1.f : ab.x;
-    bu = u < 0 ? 0.f : ab.y;
+    au = ab.x; bu = ab.y;
 }
 
 __device__ __forceinline__ void ld32(float (&v)[32], const float* __restrict__ p, bool ok)
